@@ -129,20 +129,104 @@ EMPM_HD bool viscoplastic(const M3& U, V3& s, const M3& V, float mu, float ys, f
     return true;
 }
 
+// Rotation R of the polar decomposition F = R S, by Newton's iteration
+// X <- (X + X^-T) / 2 from X = F (N. J. Higham, "Computing the polar
+// decomposition with applications", SIAM J. Sci. Stat. Comput. 7, 1986), which
+// converges quadratically: a step that moved X by less than 2e-4 leaves an
+// error below 2e-8. Returns false, without a result, for F that is inverted,
+// nearly singular or far from a rotation (or not finite).
+EMPM_HD bool polar_rotation(const M3& F, M3& R) {
+    R = F;
+#pragma unroll 1
+    for (int it = 0; it < 6; ++it) {
+        const M3 X = R;
+        M3 c;   // cofactors: X^-T = c / det X
+        c.m[0] = X.m[4] * X.m[8] - X.m[5] * X.m[7];
+        c.m[1] = X.m[5] * X.m[6] - X.m[3] * X.m[8];
+        c.m[2] = X.m[3] * X.m[7] - X.m[4] * X.m[6];
+        c.m[3] = X.m[2] * X.m[7] - X.m[1] * X.m[8];
+        c.m[4] = X.m[0] * X.m[8] - X.m[2] * X.m[6];
+        c.m[5] = X.m[1] * X.m[6] - X.m[0] * X.m[7];
+        c.m[6] = X.m[1] * X.m[5] - X.m[2] * X.m[4];
+        c.m[7] = X.m[2] * X.m[3] - X.m[0] * X.m[5];
+        c.m[8] = X.m[0] * X.m[4] - X.m[1] * X.m[3];
+        const float d = X.m[0] * c.m[0] + X.m[1] * c.m[1] + X.m[2] * c.m[2];
+        if (!(d > 0.05f && d < 20.f)) return false;
+        float h = fast_rcp(d);
+        h = 0.5f * (h + h * (1.f - d * h));   // to the last bit or so: an error here stretches R
+        float move = 0.f;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            R.m[e] = h * c.m[e] + 0.5f * X.m[e];
+            move = fmaxf(move, fabsf(R.m[e] - X.m[e]));
+        }
+        if (move < 2e-4f) return true;
+    }
+    return false;
+}
+
+// Fixed-corotated stress (mpm_utils.py:8-15) without a singular value
+// decomposition: tau = 2 mu (F - R) F^T + lam J (J - 1) I for jelly, and for
+// plasticine when F is certainly inside its yield surface, where the return map
+// changes nothing. Returns false when it does not apply (the caller then takes
+// the general update).
+//
+// The yield test compares 2 mu |dev eps| with the yield stress, eps the
+// logarithms of the singular values. With H = F^T F - I and eigenvalues l_i of
+// F^T F, |log l_i - log l_j| <= |l_i - l_j| / min l, so |dev eps| <= |dev H| /
+// (2 (1 - |H|)) in the Frobenius norm: a particle whose bound is below 0.999 of
+// its yield stress is inside. J - 1 is formed from F - I and the product with
+// (F - R)'s first-order rounding (a small rotation, antisymmetric) cancels in
+// the symmetrised product, so the result is at least as exact as through the
+// decomposition.
+EMPM_HD bool fcr_elastic(const M3& F, float mu, float lam, float ys, bool yields, M3& tau, M3& R, float& J1) {
+    if (yields) {
+        const V3 a = col(F, 0), b = col(F, 1), c = col(F, 2);
+        const float h0 = dot(a, a) - 1.f, h1 = dot(b, b) - 1.f, h2 = dot(c, c) - 1.f;
+        const float o2 = 2.f * (dot(a, b) * dot(a, b) + dot(a, c) * dot(a, c) + dot(b, c) * dot(b, c));
+        const float t = (h0 + h1 + h2) / 3.f;
+        const float full = sqrtf(h0 * h0 + h1 * h1 + h2 * h2 + o2);
+        const float dev = sqrtf((h0 - t) * (h0 - t) + (h1 - t) * (h1 - t) + (h2 - t) * (h2 - t) + o2);
+        if (!(full < 0.5f && mu * dev < 0.999f * ys * (1.f - full))) return false;
+    }
+    if (!polar_rotation(F, R)) return false;
+    const M3 D = F - R;
+    // J - 1 from E = F - I: tr E + its principal 2x2 minors + det E
+    const float e0 = F.m[0] - 1.f, e4 = F.m[4] - 1.f, e8 = F.m[8] - 1.f;
+    const float k0 = e4 * e8 - F.m[5] * F.m[7];
+    const float minors = k0 + (e0 * e8 - F.m[2] * F.m[6]) + (e0 * e4 - F.m[1] * F.m[3]);
+    const float detE = e0 * k0 - F.m[1] * (F.m[3] * e8 - F.m[5] * F.m[6]) + F.m[2] * (F.m[3] * F.m[7] - e4 * F.m[6]);
+    J1 = (e0 + e4 + e8) + (minors + detE);
+    const float p = lam * (1.f + J1) * J1, m2 = 2.f * mu;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = i; j < 3; ++j) {
+            float s = D.m[3 * i] * F.m[3 * j] + D.m[3 * i + 1] * F.m[3 * j + 1] + D.m[3 * i + 2] * F.m[3 * j + 2];
+            if (i == j) {
+                tau.m[4 * i] = m2 * s + p;
+            } else {
+                s += D.m[3 * j] * F.m[3 * i] + D.m[3 * j + 1] * F.m[3 * i + 1] + D.m[3 * j + 2] * F.m[3 * i + 2];
+                tau.m[3 * i + j] = tau.m[3 * j + i] = mu * s;
+            }
+        }
+    return true;
+}
+
 // Return map + stress for one particle. mu, lam, ys are read and, for the
 // von Mises models, updated in place.
 // MAT >= 0 compiles the update for that material only (a batch whose
 // instances all use it); -1 switches on ms.material.
 template <int MAT = -1>
-EMPM_HD ConstitutiveOut constitutive(const M3& Ft, float& mu, float& lam, float& ys, float dt,
-                                     const MaterialScalars& ms) {
+EMPM_HD ConstitutiveOut constitutive_general(const M3& Ft, float& mu, float& lam, float& ys, float dt,
+                                             const MaterialScalars& ms) {
     ConstitutiveOut out;
     out.mat_changed = false;
+    const int material = MAT >= 0 ? MAT : ms.material;
     M3 U, V;
     V3 s;
     svd3(Ft, U, s, V);
     M3 F = Ft;
-    const int material = MAT >= 0 ? MAT : ms.material;
     switch (material) {
         case 1: von_mises(U, s, V, mu, lam, ys, ms, false, out.mat_changed, F); break;
         case 2: sand(U, s, V, mu, lam, ms, F); break;
@@ -193,6 +277,54 @@ EMPM_HD ConstitutiveOut constitutive(const M3& Ft, float& mu, float& lam, float&
     out.F = F;
     out.tau = tau;
     return out;
+}
+
+// The same as a call, for kernels that take fcr_elastic first: their registers
+// are then those of the common path. io: F_trial, mu, lam, yield in; elastic F,
+// mu, lam, yield, tau and the changed mark out.
+struct ConstitutiveCall { M3 F, tau; float mu, lam, ys; int changed; };
+template <int MAT>
+#ifdef __CUDACC__
+__host__ __device__ __noinline__
+#else
+inline
+#endif
+void constitutive_call(ConstitutiveCall* io, float dt, const MaterialScalars* ms) {
+    const M3 Ft = io->F;
+    const ConstitutiveOut o = constitutive_general<MAT>(Ft, io->mu, io->lam, io->ys, dt, *ms);
+    io->F = o.F;
+    io->tau = o.tau;
+    io->changed = o.mat_changed;
+}
+
+template <int MAT = -1>
+EMPM_HD ConstitutiveOut constitutive(const M3& Ft, float& mu, float& lam, float& ys, float dt,
+                                     const MaterialScalars& ms) {
+    const int material = MAT >= 0 ? MAT : ms.material;
+    ConstitutiveOut out;
+    if (material == 0 || material == 5) {
+        out.mat_changed = false;
+        M3 R;
+        float J1;
+        if (fcr_elastic(Ft, mu, lam, ys, material == 5, out.tau, R, J1)) {
+            out.F = Ft;
+            return out;
+        }
+        ConstitutiveCall io;
+        io.F = Ft;
+        io.mu = mu;
+        io.lam = lam;
+        io.ys = ys;
+        constitutive_call<MAT>(&io, dt, &ms);
+        mu = io.mu;
+        lam = io.lam;
+        ys = io.ys;
+        out.F = io.F;
+        out.tau = io.tau;
+        out.mat_changed = io.changed != 0;
+        return out;
+    }
+    return constitutive_general<MAT>(Ft, mu, lam, ys, dt, ms);
 }
 
 }  // namespace empm

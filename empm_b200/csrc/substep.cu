@@ -1267,9 +1267,13 @@ __global__ void k_debug_stress_adjoint(const float* Ft9, const float* mu, const 
     if (p >= n) return;
     M3 Ft, gF, gS;
     for (int i = 0; i < 9; ++i) { Ft.m[i] = Ft9[9 * p + i]; gF.m[i] = gF9[9 * p + i]; gS.m[i] = gS9[9 * p + i]; }
-    SpectralEval e;
-    spectral_eval(Ft, mu[p], lam[p], ys[p], dt, ms, e);
-    const SpectralGrad g = spectral_adjoint(e, gF, gS, g_mu[p], g_lam[p], g_ys[p]);
+    M3 tau;
+    SpectralGrad g;
+    switch (ms.material) {   // as the kernels of a batch of one material
+        case 0: g = constitutive_adjoint<0>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau); break;
+        case 5: g = constitutive_adjoint<5>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau); break;
+        default: g = constitutive_adjoint<-1>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau);
+    }
     for (int i = 0; i < 9; ++i) gFt9[9 * p + i] = g.gFt.m[i];
     g_mu[p] = g.g_mu;
     g_lam[p] = g.g_lam;
