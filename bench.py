@@ -1428,11 +1428,11 @@ def main():
     ap.add_argument("--grid", type=int, default=None, help="override the workload's grid resolution")
     ap.add_argument("--substeps", type=int, default=None, help="override the workload's substeps per step")
     ap.add_argument("--sort-every", dest="sort_every", type=int, default=None)
-    ap.add_argument("--p2g-mode", dest="p2g_mode", type=int, default=None, help="0 direct, 1 tile, 2 warp-aggregated")
+    ap.add_argument("--p2g-mode", dest="p2g_mode", type=int, default=None, help="0 direct, 1 tile, 2 summed per cell")
     ap.add_argument("--g2p-tile", dest="g2p_tile", type=int, default=None)
     ap.add_argument("--tile-cap", dest="tile_cap", type=int, default=None)
     ap.add_argument("--seg-cap", dest="seg_cap", type=int, default=None,
-                    help="warp-aggregated P2G: longest same-cell run per reduction (4, 8, 16, 32)")
+                    help="G2P adjoint: longest same-cell run per reduction (4, 8, 16, 32)")
     ap.add_argument("--fuse", dest="fuse", type=int, default=None,
                     help="1 = fused G2P + stress + P2G between cell sorts (default), 0 = separate kernels")
     ap.add_argument("--resume-blocks", dest="resume_blocks", type=int, default=None,

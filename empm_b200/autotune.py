@@ -6,9 +6,9 @@ the FP64 oracle), so it can be picked by speed alone. The tuner times a few
 substeps of the caller's own workload under each candidate:
 
 * ``sort_every``: the period of the cell sort (8, 16, 32 substeps);
-* ``p2g_mode`` / ``tile_cap`` / ``seg_cap``: warp-aggregated reductions into
-  the grid over same-cell runs of at most 4 or 8 lanes, or accumulation in a
-  per-CTA shared-memory node tile of 512 / 1024 / 2048 nodes (the tile shape);
+* ``p2g_mode`` / ``tile_cap`` / ``seg_cap``: contributions summed per cell, or
+  accumulation in a per-CTA shared-memory node tile of 512 / 1024 / 2048 nodes
+  (the tile shape); the longest same-cell run of the G2P adjoint, 4 or 8 lanes;
 * ``g2p_tile``: G2P gathering directly from L2 or from a staged tile;
 * ``fuse``: the G2P of each substep and the stress + P2G of the next as one
   kernel between cell sorts, or separate kernels.
@@ -30,7 +30,7 @@ CANDIDATES: List[Dict[str, int]] = [
     dict(sort_every=s, p2g_mode=m, tile_cap=c, seg_cap=k, g2p_tile=g, fuse=f)
     for s, (m, c, k), g, f in itertools.product(
         (8, 16, 32), ((2, 1024, 4), (2, 1024, 8), (1, 512, 4), (1, 1024, 4), (1, 2048, 4)), (0, 1), (1, 0))
-    if f == 1 or (m == 2 and g == 0)   # fusing applies to warp-aggregated P2G with direct G2P only
+    if f == 1 or (m == 2 and g == 0)   # fusing applies to the per-cell P2G with direct G2P only
 ]
 OPTION_NAMES = ("sort_every", "p2g_mode", "tile_cap", "seg_cap", "g2p_tile", "fuse")
 DEFAULTS = dict(sort_every=32, p2g_mode=2, tile_cap=1024, seg_cap=4, g2p_tile=0, fuse=1)

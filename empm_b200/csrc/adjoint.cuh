@@ -81,7 +81,7 @@ struct AdjG2PArgs {
 //
 // Lanes whose particles share an instance and base cell (contiguous in cell
 // order) sum their node-velocity adjoints with shuffles; the segment head
-// issues one reduction per node, as k_p2g_warpagg does for the momentum.
+// issues one reduction per node.
 // Every lane of the warp runs the node loop, invalid lanes with zeros.
 // ROUNDS < 5: runs are capped at 2^ROUNDS lanes (a.seg_cap equals it), so the
 // shuffle rounds the cap never needs are not compiled in; ROUNDS 5 takes any
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128, EMPM_ADJ_G2P_MIN_CTAS) k_adj_g2p(const Ad
     const int ui = __shfl_up_sync(0xffffffffu, inst, 1);
     const bool run_head = lane == 0 || uv != (int)valid || ui != inst || u0 != b0 || u1 != b1 || u2 != b2;
     // runs longer than seg_cap (a power of two) get another head every seg_cap
-    // lanes, as in k_p2g_warpagg
+    // lanes
     const unsigned run_heads = __ballot_sync(0xffffffffu, run_head);
     const int run_start = 31 - __clz(run_heads & (0xffffffffu >> (31 - lane)));
     const bool head = run_head || ((lane - run_start) & (seg_cap - 1)) == 0;

@@ -12,9 +12,9 @@
 // Launch paths:
 //   * direct: one particle per thread, 16-byte vector reductions into the grid;
 //   * sorted (rollouts): particles in cell order, re-sorted every few substeps;
-//     P2G sums the contributions of same-cell particles of a warp with
-//     shuffles and issues one reduction per cell and node (default), or
-//     accumulates per chunk in a shared-memory node tile (option);
+//     P2G sums the contributions of same-cell particles of a warp and issues one
+//     reduction per cell and node (default, cellsum.cuh), or accumulates per
+//     chunk in a shared-memory node tile (option);
 //     G2P gathers directly or from a staged shared-memory tile (option);
 //   * the grid update visits only the 4^3 node blocks that P2G touched.
 #pragma once
@@ -22,36 +22,25 @@
 #include "../../include/empm_b200.h"
 #include "grid.cuh"
 #include "substep.cuh"
+#include "cellsum.cuh"
 
-// Minimum resident CTAs per SM asked of the compiler for the two particle
-// kernels of the sorted path (register caps: 65536 / (threads x CTAs)).
+// Threads per CTA of the particle kernels that scatter per cell, and the
+// minimum resident CTAs per SM asked of the compiler: for stress + P2G (at 5: 96
+// registers, 46 us for 500k particles; at 4 51 us), with the G2P before it (at 4:
+// 128 registers, no spills, 64.5 us and 371 us on the population; at 5 68.5 and
+// 379 us, at 6 72 and 390 us; CTAs of 256 threads 5-10 % slower), and for G2P alone
+// (CTAs of 128).
+#ifndef EMPM_CELL_THREADS
+#define EMPM_CELL_THREADS 128
+#endif
 #ifndef EMPM_P2G_MIN_CTAS
-#define EMPM_P2G_MIN_CTAS 4
+#define EMPM_P2G_MIN_CTAS 5
 #endif
-#ifndef EMPM_G2P_MIN_CTAS
-#define EMPM_G2P_MIN_CTAS 8
-#endif
-// ... and for the fused G2P + stress + P2G kernel
 #ifndef EMPM_FUSED_MIN_CTAS
 #define EMPM_FUSED_MIN_CTAS 4
 #endif
-// 1: each warp of the fused kernel first copies the grid nodes its lanes'
-// stencils cover (their bounding box, at most EMPM_WARP_TILE_NODES nodes) into
-// shared memory and gathers from there; warps whose box is larger, leaves the
-// grid or spans two instances gather from global memory. Measured on the
-// population workload it is slower than gathering through L1 (648 us per
-// launch with 128-node boxes, 613 us with 192, against 595 us), so it is off.
-#ifndef EMPM_FUSED_WARP_TILE
-#define EMPM_FUSED_WARP_TILE 0
-#endif
-#ifndef EMPM_WARP_TILE_NODES
-#define EMPM_WARP_TILE_NODES 128
-#endif
-// 1: the fused kernel's G2P gathers with a run-time outer stencil loop
-// (population workload: 598 us per launch against 604 us fully unrolled; at 3
-// or 2 CTAs per SM 603-608 and 722 us)
-#ifndef EMPM_FUSED_G2P_LOOP
-#define EMPM_FUSED_G2P_LOOP 1
+#ifndef EMPM_G2P_MIN_CTAS
+#define EMPM_G2P_MIN_CTAS 8
 #endif
 
 namespace empm {
@@ -502,35 +491,169 @@ struct GlobalFetch {
     }
 };
 
-// Node velocities from a warp's shared-memory copy of the nodes its lanes'
-// stencils cover: a box with origin o and extents e (tile index
-// ((i - o0) * e1 + (j - o1)) * e2 + (k - o2)). The outer axis may be a run-time
-// index (g2p_gather_rt), so its term is formed per call.
-struct WarpTileFetch {
-    const float4* tile;
-    int o0, o1, o2, e1, e2;
-    struct Bound {
-        const float4* tile;
-        int x0, e12;
-        int y[3], z[3];
-        __device__ __forceinline__ V3 operator()(int i, int j, int k) const {
-            const float4 g = tile[x0 + i * e12 + y[j] + z[k]];
-            return v3(g.x, g.y, g.z);
-        }
-    };
-    __device__ __forceinline__ Bound bind(const Stencil& st, bool) const {
-        Bound b;
-        b.tile = tile;
-        b.e12 = e1 * e2;
-        b.x0 = (st.b[0] - o0) * b.e12;
+// G2P gather of a stencil inside the grid, factorised over the inner axis: per
+// row (i, j) the three nodes are combined with wz, dwz and k wz first, then the
+// rows with weights in x and y; x and y components travel as pairs.
+__device__ __forceinline__ G2POut g2p_gather_rows(const int b[3], const float fx[3], float inv_dx, int boff, int NB,
+                                                  const float4* __restrict__ vel) {
+    P3 V = p3_zero(), M0 = V, M1 = V, M2 = V;   // sum wg, and its moments in i, j, k
+    P3 g0 = V, g1 = V, g2 = V;                  // columns of sum grid_v (x) dweight / inv_dx
+    F2 wz[3], uz[3];
+    unsigned zpart[3];
 #pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            b.y[o] = (st.b[1] + o - o1) * e2;
-            b.z[o] = st.b[2] + o - o2;
-        }
-        return b;
+    for (int k = 0; k < 3; ++k) {
+        float w, u;
+        bspline_at(fx[2], k, w, u);
+        wz[k] = f2_both(w);
+        uz[k] = f2_both(u);
+        zpart[k] = ((unsigned)((b[2] + k) >> 2) << 6) | ((b[2] + k) & 3);
     }
-};
+    const F2 kz2 = f2_add(wz[2], wz[2]);
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        float wx, ux;
+        bspline_at(fx[0], i, wx, ux);
+        const int ix = b[0] + i;
+        const int xblk = boff + (ix >> 2) * NB * NB;
+        const unsigned xoff = (ix & 3) << 4;
+        P3 Vi = p3_zero();
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int iy = b[1] + j;
+            const unsigned row = ((unsigned)(xblk + (iy >> 2) * NB) << 6) + (xoff | ((iy & 3) << 2));
+            const float4 a0 = __ldg(vel + (row + zpart[0])), a1 = __ldg(vel + (row + zpart[1])),
+                         a2 = __ldg(vel + (row + zpart[2]));
+            const P3 n0 = p3(f2_make(a0.x, a0.y), a0.z), n1 = p3(f2_make(a1.x, a1.y), a1.z),
+                     n2 = p3(f2_make(a2.x, a2.y), a2.z);
+            float wy, uy;
+            bspline_at(fx[1], j, wy, uy);
+            const F2 wxy = f2_both(wx * wy);
+            const P3 T0 = p3_fma(wz[2], n2, p3_fma(wz[1], n1, p3_mul(wz[0], n0)));
+            const P3 T1 = p3_fma(uz[2], n2, p3_fma(uz[1], n1, p3_mul(uz[0], n0)));
+            const P3 Tk = p3_fma(kz2, n2, p3_mul(wz[1], n1));
+            Vi = p3_fma(wxy, T0, Vi);
+            if (j == 1) M1 = p3_fma(wxy, T0, M1);
+            if (j == 2) M1 = p3_fma(f2_add(wxy, wxy), T0, M1);
+            M2 = p3_fma(wxy, Tk, M2);
+            g0 = p3_fma(f2_both(ux * wy), T0, g0);
+            g1 = p3_fma(f2_both(wx * uy), T0, g1);
+            g2 = p3_fma(wxy, T1, g2);
+        }
+        V = p3_add(V, Vi);
+        M0 = p3_fma(f2_both((float)i), Vi, M0);
+    }
+    G2POut o;
+    o.v.z = V.z;
+    f2_split(V.xy, o.v.x, o.v.y);
+    const P3 mc[3] = {M0, M1, M2}, gc[3] = {g0, g1, g2};
+    const float c4 = 4.f * inv_dx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        float x, y;
+        f2_split(mc[c].xy, x, y);
+        o.C.m[c] = c4 * (x - fx[c] * o.v.x);
+        o.C.m[3 + c] = c4 * (y - fx[c] * o.v.y);
+        o.C.m[6 + c] = c4 * (mc[c].z - fx[c] * o.v.z);
+        f2_split(gc[c].xy, x, y);
+        o.gradv.m[c] = inv_dx * x;
+        o.gradv.m[3 + c] = inv_dx * y;
+        o.gradv.m[6 + c] = inv_dx * gc[c].z;
+    }
+    return o;
+}
+
+// The same for a stencil that leaves the grid: nodes outside read as zero.
+__device__ __noinline__ void g2p_gather_edge(G2POut* o, float x, float y, float z, float inv_dx, int boff, int NB,
+                                             int G, const float4* vel) {
+    const Stencil st = make_stencil(v3(x, y, z), inv_dx);
+    const GlobalFetch::Bound fetch{vel, stencil_addr(boff, NB, st.b), st.b, G, false};
+    *o = g2p_gather_rt(st, inv_dx, fetch);
+}
+
+// ---- fetching ahead ---------------------------------------------------------
+// With 16 warps per SM the gather's waits are not hidden behind other warps, and
+// the particle's F and material would be waited for once more after it. They are
+// sent for before the gather, straight into the thread's part of the scatter's
+// shared memory (cp.async), which is free until then (population fused kernel
+// 397 -> 371 us; sending for the nodes of the warp's cells as well, to share them
+// there: 362 us, but 66.3 against 64.5 us for 500k particles at 4 per cell).
+__device__ __forceinline__ void copy_ahead16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void copy_ahead4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+struct Ahead { M3 F; float mu, lam, ys, vol; };
+
+template <int NT>
+__device__ __forceinline__ void particle_ahead(CellScatter<true, NT>& sh, const F9Planes& F, const MaterialArrays& M,
+                                               int p) {
+    const int t = threadIdx.x;
+    copy_ahead16(&sh.q[0][t], F.a + p);
+    copy_ahead16(&sh.q[1][t], F.b + p);
+    copy_ahead4(&sh.q[2][t].x, F.c + p);
+    copy_ahead4(&sh.q[2][t].y, M.mu + p);
+    copy_ahead4(&sh.q[2][t].z, M.lam + p);
+    copy_ahead4(&sh.q[2][t].w, M.ys + p);
+    copy_ahead4(&sh.q[3][t].x, M.vol + p);
+}
+
+template <int NT>
+__device__ __forceinline__ Ahead particle_arrived(const CellScatter<true, NT>& sh) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const int t = threadIdx.x;
+    const float4 a = sh.q[0][t], b = sh.q[1][t], m = sh.q[2][t];
+    Ahead r;
+    r.F.m[0] = a.x; r.F.m[1] = a.y; r.F.m[2] = a.z; r.F.m[3] = a.w;
+    r.F.m[4] = b.x; r.F.m[5] = b.y; r.F.m[6] = b.z; r.F.m[7] = b.w;
+    r.F.m[8] = m.x;
+    r.mu = m.y;
+    r.lam = m.z;
+    r.ys = m.w;
+    r.vol = sh.q[3][t].x;
+    return r;
+}
+
+// G2P of particle p at (x, mass) = xm: its gathered velocity and affine matrix
+// are returned, nx is the clamped new position, Fn the new trial F and ah what was
+// fetched ahead for it; status bits are set.
+template <int NT>
+__device__ __forceinline__ G2POut g2p_move(CellScatter<true, NT>& sh, const StepConsts& c, float dt, float4 xm,
+                                           const F9Planes& Fe, const MaterialArrays& M, int p, const float4* vel,
+                                           V3& nx, M3& Fn, Ahead& ah) {
+    particle_ahead(sh, Fe, M, p);
+    const float xs[3] = {xm.x, xm.y, xm.z};
+    int b[3];
+    float fx[3];
+    bool in_grid = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        b[a] = base_node(xs[a], c.inv_dx);
+        fx[a] = base_frac(xs[a], c.inv_dx, b[a]);
+        in_grid = in_grid && b[a] >= 0 && b[a] + 2 < c.G;
+    }
+    G2POut o;
+    if (in_grid) {
+        o = g2p_gather_rows(b, fx, c.inv_dx, c.boff, c.NB, vel);
+    } else {
+        G2POut e;
+        g2p_gather_edge(&e, xm.x, xm.y, xm.z, c.inv_dx, c.boff, c.NB, c.G, vel);
+        o = e;
+    }
+    const float dx = 1.f / c.inv_dx;
+    const float lo = dx * 2.f, hi = c.grid_lim - dx * 2.f;
+    nx = v3(xm.x, xm.y, xm.z) + dt * o.v;
+    nx = v3(fminf(fmaxf(nx.x, lo), hi), fminf(fmaxf(nx.y, lo), hi), fminf(fmaxf(nx.z, lo), hi));
+    ah = particle_arrived(sh);
+    Fn = (m3_identity() + dt * o.gradv) * ah.F;
+    unsigned bad = 0;
+    if (!finite3(o.v) || !finite3(nx) || !isfinite(Fn.m[0] + Fn.m[4] + Fn.m[8])) bad |= EMPM_STATUS_NAN;
+    if (fmaxf(fmaxf(fabsf(o.v.x), fabsf(o.v.y)), fabsf(o.v.z)) * dt > dx) bad |= EMPM_STATUS_CFL;
+    if (!in_grid) bad |= EMPM_STATUS_OUT_OF_BAND;
+    if (bad) atomicOr(c.status, bad);
+    return o;
+}
 
 __global__ void __launch_bounds__(128, EMPM_G2P_MIN_CTAS) k_g2p_direct(ParticleArrays P, F9Planes Fe, MaterialArrays M,
                                                     ParticleArrays out, Launch L, const float4* vel) {
@@ -666,94 +789,74 @@ __global__ void k_unsort(const UnsortArgs a) {
 }
 
 // -------------------------------------------------------------------------
-// sorted path, default P2G: warp-aggregated reductions
+// sorted path, default P2G: contributions summed per cell (cellsum.cuh)
 // -------------------------------------------------------------------------
-// Lanes whose particles share an instance and base cell form a contiguous
-// segment of the warp (cell-sorted order); for each of the 27 stencil nodes
-// the segment's contributions are summed with shuffles and only the segment
-// head issues the 16-byte reduction to the grid.
-//
-// Same-cell runs are split every seg_cap = 2^ROUNDS lanes, so a segment sums
-// in at most ROUNDS shuffle rounds; the rounds a run cap never needs are not
-// compiled in (smaller code for the instruction cache).
-// The warp-aggregated scatter of one prepared particle per lane (all 32
-// lanes of the warp take part; lanes with valid == false contribute zeros and
-// never write). c: the lane's instance constants for this substep.
-template <int ROUNDS>
-__device__ __forceinline__ void warpagg_scatter(bool valid, int inst, const P2GParticle& q, const StepConsts& c,
-                                                float4* grid, unsigned char* flags) {
-    constexpr int seg_cap = 1 << ROUNDS;
-    const int lane = threadIdx.x & 31;
-    // a segment is a run of lanes with the same validity, instance and base
-    // cell; lanes without a particle contribute zeros and never write
-    const int b0 = valid ? q.st.b[0] : lane, b1 = valid ? q.st.b[1] : 0, b2 = valid ? q.st.b[2] : 0;
-    const int u0 = __shfl_up_sync(0xffffffffu, b0, 1), u1 = __shfl_up_sync(0xffffffffu, b1, 1),
-              u2 = __shfl_up_sync(0xffffffffu, b2, 1);
-    const int uv = __shfl_up_sync(0xffffffffu, (int)valid, 1);
-    const int ui = __shfl_up_sync(0xffffffffu, inst, 1);
-    const bool run_head = lane == 0 || uv != (int)valid || ui != inst || u0 != b0 || u1 != b1 || u2 != b2;
-    // runs longer than seg_cap (a power of two) get another head every
-    // seg_cap lanes: fewer shuffle rounds below, more reductions into the grid
-    const unsigned run_heads = __ballot_sync(0xffffffffu, run_head);
-    const int run_start = 31 - __clz(run_heads & (0xffffffffu >> (31 - lane)));
-    const bool head = run_head || ((lane - run_start) & (seg_cap - 1)) == 0;
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const unsigned above = lane == 31 ? 0u : (heads & (0xffffffffu << (lane + 1)));
-    const int end = above ? (__ffs(above) - 2) : 31;
-    const int seglen = head ? end - lane + 1 : 1;
-    const int maxlen = __reduce_max_sync(0xffffffffu, seglen);
-    const int G = c.G;
-    const bool in_grid = valid && stencil_in_grid(q.st, G);
-    if (valid && !in_grid) atomicOr(c.status, EMPM_STATUS_OUT_OF_BAND);
-    P2GPre pre;
+// Stress and scatter of a CTA's particles; every thread takes part. A thread
+// with valid set has particle p at x with velocity v, affine matrix C and trial F
+// Ft: velocity modifiers, return map and stress are applied, the elastic F, the
+// material scalars when they change and (v_out not NULL) the velocity after the
+// modifiers are written, and the contributions
+//   (weight * mass) (v + C dpos) - dt vol stress dweight, dpos = ((i, j, k) - fx) dx,
+// go into the grid: a = v - dx C fx, B = dx C and S = -dt inv_dx vol stress.
+template <int MAT, int NT>
+__device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid, const StepConsts& c,
+                                          const EmpmStep& sp, const MaterialArrays& M, int p, V3 x, float mass, V3 v,
+                                          const M3& C, const M3& Ft, float mu, float lam, float ys, float vol,
+                                          const F9Planes& Fe, float4* v_out, float4* grid, unsigned char* flags) {
+    const float xs[3] = {x.x, x.y, x.z};
+    int b[3] = {0, 0, 0};
+    if (valid)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) b[a] = base_node(xs[a], c.inv_dx);
+    const CellSlot cell = cell_scatter_slot(sh, valid, b, c.G, c.NB, c.boff);
     if (valid) {
-        pre = p2g_pre(q, c.dx, c.inv_dx, c.step->dt);
-    } else {
-        pre.st = make_stencil(v3(0.f, 0.f, 0.f), 1.f);
-        pre.m = 0.f;
-        pre.a = v3(0.f, 0.f, 0.f);
-        pre.B = m3_zero();
-        pre.S = m3_zero();
-    }
-    // The reduction rounds are unrolled: each is skipped by a warp-uniform
-    // branch once 2^r >= maxlen, and the per-lane "partner inside my segment"
-    // tests are formed once instead of per node. The node address is formed
-    // only in the head lanes (keeping precomputed per-axis address terms live
-    // across the 27 nodes measured slower here).
-    unsigned take = 0;
-#pragma unroll
-    for (int r = 0; r < ROUNDS; ++r) take |= lane + (1 << r) <= end ? 1u << r : 0u;
-    p2g_emit(pre, [&](int i, int j, int k, float4 v) {
-#pragma unroll
-        for (int r = 0; r < ROUNDS; ++r) {
-            const int d = 1 << r;
-            if (d < maxlen) {
-                const float tx = __shfl_down_sync(0xffffffffu, v.x, d);
-                const float ty = __shfl_down_sync(0xffffffffu, v.y, d);
-                const float tz = __shfl_down_sync(0xffffffffu, v.z, d);
-                const float tw = __shfl_down_sync(0xffffffffu, v.w, d);
-                if (take & (1u << r)) { v.x += tx; v.y += ty; v.z += tz; v.w += tw; }
-            }
+        if (sp.n_modifiers > 0) {
+            const int mi = M.pid ? __ldg(M.pid + p) : p;
+            apply_modifiers(sp, mi, x, mass, v);
         }
-        if (head && valid && (in_grid || node_in_grid(q.st.b, i, j, k, G)))
-            red_add_v4(grid + gaddr(c, q.st.b[0] + i, q.st.b[1] + j, q.st.b[2] + k), v);
-    });
-    if (head && valid) mark_stencil_blocks(flags, q.st, c);
+        if (v_out) v_out[p] = make_float4(v.x, v.y, v.z, 0.f);
+        float fx[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) fx[a] = base_frac(xs[a], c.inv_dx, b[a]);
+        const M3 B = (mass * c.dx) * damp_affine(C, c.rpic);
+        cell_scatter_put(sh, cell.slot, fx, mass, mass * v - B * v3(fx[0], fx[1], fx[2]), B);
+        const ConstitutiveOut co = constitutive<MAT>(Ft, mu, lam, ys, sp.dt, *c.ms);
+        f9_store(Fe, p, co.F);
+        if (co.mat_changed) { M.mu[p] = mu; M.lam[p] = lam; M.ys[p] = ys; }
+        cell_scatter_put(sh, cell.slot, (sp.dt * c.inv_dx * -vol) * co.tau);
+        if (cell.base < 0) {
+            atomicOr(c.status, EMPM_STATUS_OUT_OF_BAND);
+            cell_scatter_edge(&sh, cell.slot, b[0], b[1], b[2], c.G, c.NB, c.boff, grid, flags);
+        }
+    }
+    cell_scatter(sh, cell, grid, flags);
 }
 
-// Same-cell runs are split every seg_cap = 2^ROUNDS lanes, so a segment sums
-// in at most ROUNDS shuffle rounds; the rounds a run cap never needs are not
-// compiled in (smaller code for the instruction cache).
-template <int ROUNDS, int MAT = -1>
-__global__ void __launch_bounds__(256, EMPM_P2G_MIN_CTAS) k_p2g_warpagg(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
-                                                     float4* grid, unsigned char* flags) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int inst = p < L.n_total ? find_instance_particle(L, p) : 0;
-    const StepConsts c = consts_of(L, inst);
-    P2GParticle q;
-    bool valid = false;
-    if (p < L.n_total) valid = prepare_particle<MAT>(P, M, Fe, c, p, q);
-    warpagg_scatter<ROUNDS>(valid, inst, q, c, grid, flags);
+template <int NT, int MAT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
+                                                        float4* grid, unsigned char* flags) {
+    __shared__ CellScatter<true, NT> sh;
+    cell_scatter_begin(sh);
+    const int p = blockIdx.x * NT + threadIdx.x;
+    const StepConsts c = consts_of(L, p < L.n_total ? find_instance_particle(L, p) : 0);
+    const EmpmStep& sp = *c.step;
+    // a held instance contributes nothing this substep
+    const bool valid = p < L.n_total && !(M.sel && __ldg(M.sel + p) != 0) && !sp.hold;
+    float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vv = xm;
+    M3 C = m3_zero(), F = C;
+    float mu = 0.f, lam = 0.f, ys = 0.f, vol = 0.f;
+    if (valid) {
+        xm = __ldg(P.x + p);
+        vv = __ldg(P.v + p);
+        C = f9_load(P.C, p);
+        F = f9_load(P.F, p);
+        mu = __ldg(M.mu + p);
+        lam = __ldg(M.lam + p);
+        ys = __ldg(M.ys + p);
+        vol = __ldg(M.vol + p);
+    }
+    p2g_cells<MAT>(sh, valid, c, sp, M, p, v3(xm.x, xm.y, xm.z), xm.w, v3(vv.x, vv.y, vv.z), C, F, mu, lam, ys, vol,
+                   Fe, sp.n_modifiers > 0 ? P.v : nullptr, grid, flags);
 }
 
 // -------------------------------------------------------------------------
@@ -771,131 +874,37 @@ __global__ void __launch_bounds__(256, EMPM_P2G_MIN_CTAS) k_p2g_warpagg(Particle
 // full state. Held instances (step-table hold) must stay held once held within
 // the run: when a particle's instance becomes held at substep s, its state
 // after the G2P of s-1 is written in full, then left alone.
-// MINB: resident CTAs per SM asked of the compiler. Launches over few
-// particles (CTAs of 64 threads, a few warps per SM) use MINB = 1: registers
-// are then not what limits them, so the kernel keeps all its state in
-// registers and gathers with the unrolled loop (C1, 20k particles: 25.3 ->
-// 23.7 us per substep).
-template <int ROUNDS, int MAT = -1, int MINB = EMPM_FUSED_MIN_CTAS>
-__global__ void __launch_bounds__(256, MINB) k_g2p2g(ParticleArrays P, MaterialArrays M, F9Planes Fe,
-                                                                  Launch L, int g2p_table, const float4* vel,
-                                                                  float4* mom, unsigned char* flags) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+template <int NT, int MAT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_g2p2g(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
+                                                    int g2p_table, const float4* vel, float4* mom,
+                                                    unsigned char* flags) {
+    __shared__ CellScatter<true, NT> sh;
+    cell_scatter_begin(sh);
+    const int p = blockIdx.x * NT + threadIdx.x;
     const int inst = p < L.n_total ? find_instance_particle(L, p) : 0;
     const StepConsts c = consts_of(L, inst);   // substep s: stress + P2G
-    P2GParticle q;
-    bool valid = false;
-    // which lanes run the G2P of substep s-1 (simulated, not held)
-    bool g_on = false;
-    float4 xm = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p < L.n_total && !(M.sel && __ldg(M.sel + p) != 0)) {
-        g_on = !L.steps[(size_t)g2p_table * L.n_inst + inst].hold;
-        if (g_on) xm = __ldg(P.x + p);
-    }
-#if EMPM_FUSED_WARP_TILE
-    // the warp's stencil nodes into shared memory (all lanes take part)
-    __shared__ float4 s_tile[256 / 32][EMPM_WARP_TILE_NODES];
-    const int wlane = threadIdx.x & 31;
-    float4* wtile = s_tile[threadIdx.x >> 5];
-    int gb[3] = {0, 0, 0};
-    if (g_on) {
-        gb[0] = base_node(xm.x, c.inv_dx);
-        gb[1] = base_node(xm.y, c.inv_dx);
-        gb[2] = base_node(xm.z, c.inv_dx);
-    }
-    const unsigned g_lanes = __ballot_sync(0xffffffffu, g_on);
-    int box_o[3], box_e[3];
-    bool tiled = false;
-    if (g_lanes) {
-        int hi[3];
-#pragma unroll
-        for (int a3 = 0; a3 < 3; ++a3) {
-            box_o[a3] = __reduce_min_sync(0xffffffffu, g_on ? gb[a3] : INT_MAX);
-            hi[a3] = __reduce_max_sync(0xffffffffu, g_on ? gb[a3] : INT_MIN);
-            box_e[a3] = hi[a3] - box_o[a3] + 3;
-        }
-        const int imin = __reduce_min_sync(0xffffffffu, g_on ? inst : INT_MAX);
-        const int imax = __reduce_max_sync(0xffffffffu, g_on ? inst : INT_MIN);
-        const int leader = __ffs(g_lanes) - 1;
-        const int Gw = __shfl_sync(0xffffffffu, c.G, leader);
-        const int NBw = __shfl_sync(0xffffffffu, c.NB, leader);
-        const int boffw = __shfl_sync(0xffffffffu, c.boff, leader);
-        const int count = box_e[0] * box_e[1] * box_e[2];
-        tiled = imin == imax && count <= EMPM_WARP_TILE_NODES && box_o[0] >= 0 && box_o[1] >= 0 &&
-                box_o[2] >= 0 && hi[0] + 2 < Gw && hi[1] + 2 < Gw && hi[2] + 2 < Gw;
-        if (tiled) {
-            const int e12 = box_e[1] * box_e[2];
-            for (int t = wlane; t < count; t += 32) {
-                const int ti = t / e12, tr = t - ti * e12;
-                const int tj = tr / box_e[2], tk = tr - tj * box_e[2];
-                const int gi = box_o[0] + ti, gj = box_o[1] + tj, gk = box_o[2] + tk;
-                const long long addr = ((long long)(boffw + block_of(gi, gj, gk, NBw)) << 6) | ((gi & 3) << 4) |
-                                       ((gj & 3) << 2) | (gk & 3);
-                wtile[t] = __ldg(vel + addr);
-            }
-        }
-        __syncwarp();
-    }
-#endif
-    if (g_on) {
-        {
-            const EmpmStep& sg = L.steps[(size_t)g2p_table * L.n_inst + inst];   // substep s-1: G2P
-            const float dt = sg.dt;
-            const V3 x = v3(xm.x, xm.y, xm.z);
-            const Stencil st = make_stencil(x, c.inv_dx);
-            const bool in_grid = stencil_in_grid(st, c.G);
-#if EMPM_FUSED_WARP_TILE
-            G2POut o;
-            if (tiled) {
-                const WarpTileFetch fetch{wtile, box_o[0], box_o[1], box_o[2], box_e[1], box_e[2]};
-                o = g2p_gather_rt(st, c.inv_dx, fetch.bind(st, in_grid));
-            } else {
-                const GlobalFetch fetch{vel, &c};
-                o = g2p_gather_rt(st, c.inv_dx, fetch.bind(st, in_grid));
-            }
-#else
-            GlobalFetch fetch{vel, &c};
-            G2POut o;
-            if (EMPM_FUSED_G2P_LOOP && MINB > 1) o = g2p_gather_rt(st, c.inv_dx, fetch.bind(st, in_grid));
-            else o = g2p_gather(st, c.inv_dx, fetch.bind(st, in_grid));
-#endif
-            const float dx = 1.f / c.inv_dx;   // as g2p_particle computes it
-            const float lo = dx * 2.f, hi = c.grid_lim - dx * 2.f;
-            V3 nx = x + dt * o.v;
-            nx = v3(fminf(fmaxf(nx.x, lo), hi), fminf(fmaxf(nx.y, lo), hi), fminf(fmaxf(nx.z, lo), hi));
-            const M3 Fn = (m3_identity() + dt * o.gradv) * f9_load(Fe, p);
-            P.x[p] = make_float4(nx.x, nx.y, nx.z, xm.w);
-            unsigned bad = 0;
-            if (!finite3(o.v) || !finite3(nx) || !isfinite(Fn.m[0] + Fn.m[4] + Fn.m[8])) bad |= EMPM_STATUS_NAN;
-            if (fmaxf(fmaxf(fabsf(o.v.x), fabsf(o.v.y)), fabsf(o.v.z)) * dt > dx) bad |= EMPM_STATUS_CFL;
-            if (!in_grid) bad |= EMPM_STATUS_OUT_OF_BAND;
-            if (bad) atomicOr(c.status, bad);
-            const EmpmStep& sp = *c.step;
-            if (sp.hold) {
-                // held from substep s on: keep the state after this G2P
-                P.v[p] = make_float4(o.v.x, o.v.y, o.v.z, 0.f);
-                f9_store(P.C, p, o.C);
-                f9_store(P.F, p, Fn);
-            } else {
-                V3 v = o.v;
-                if (sp.n_modifiers > 0) {
-                    const int mi = M.pid ? __ldg(M.pid + p) : p;
-                    apply_modifiers(sp, mi, nx, xm.w, v);
-                }
-                float mu = __ldg(M.mu + p), lam = __ldg(M.lam + p), ys = __ldg(M.ys + p);
-                const ConstitutiveOut co = constitutive<MAT>(Fn, mu, lam, ys, sp.dt, *c.ms);
-                f9_store(Fe, p, co.F);
-                if (co.mat_changed) { M.mu[p] = mu; M.lam[p] = lam; M.ys[p] = ys; }
-                q.st = make_stencil(nx, c.inv_dx);
-                q.wm_scale = xm.w;
-                q.v = v;
-                q.Cd = damp_affine(o.C, c.rpic);
-                q.Sv = (-__ldg(M.vol + p)) * co.tau;
-                valid = true;
-            }
+    const EmpmStep& sg = L.steps[(size_t)g2p_table * L.n_inst + inst];   // substep s-1: G2P
+    const EmpmStep& sp = *c.step;
+    // lanes that run the G2P of substep s-1: simulated, not held
+    bool valid = p < L.n_total && !(M.sel && __ldg(M.sel + p) != 0) && !sg.hold;
+    const float4 xm = valid ? __ldg(P.x + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    V3 nx;
+    M3 Fn;
+    Ahead ah;
+    G2POut o;
+    if (valid) {
+        o = g2p_move(sh, c, sg.dt, xm, Fe, M, p, vel, nx, Fn, ah);
+        P.x[p] = make_float4(nx.x, nx.y, nx.z, xm.w);
+        if (sp.hold) {
+            // held from substep s on: keep the state after this G2P
+            valid = false;
+            P.v[p] = make_float4(o.v.x, o.v.y, o.v.z, 0.f);
+            f9_store(P.C, p, o.C);
+            f9_store(P.F, p, Fn);
         }
     }
-    warpagg_scatter<ROUNDS>(valid, inst, q, c, mom, flags);
+    p2g_cells<MAT>(sh, valid, c, sp, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, Fe, nullptr, mom,
+                   flags);
 }
 
 // Stored segments of a differentiable rollout (cell-sorted): the G2P of
@@ -915,137 +924,83 @@ struct SegmentStoreArgs {
     long long      np;
 };
 
-template <int ROUNDS, int MAT = -1, int MINB = EMPM_FUSED_MIN_CTAS>
-__global__ void __launch_bounds__(256, MINB) k_g2p2g_store(MaterialArrays M, Launch L, int g2p_table,
-                                                                        const float4* vel, float4* mom,
-                                                                        unsigned char* flags, SegmentStoreArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+template <int NT, int MAT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_g2p2g_store(MaterialArrays M, Launch L, int g2p_table,
+                                                          const float4* vel, float4* mom, unsigned char* flags,
+                                                          SegmentStoreArgs a) {
+    __shared__ CellScatter<true, NT> sh;
+    cell_scatter_begin(sh);
+    const int p = blockIdx.x * NT + threadIdx.x;
     const int inst = p < L.n_total ? find_instance_particle(L, p) : 0;
     const StepConsts c = consts_of(L, inst);   // substep k: stress + P2G
-    P2GParticle q;
-    bool valid = false;
-    if (p < L.n_total) {
-        const float mu0 = __ldg(M.mu + p), lam0 = __ldg(M.lam + p), ys0 = __ldg(M.ys + p);
-        a.snap[p] = mu0;
-        a.snap[a.np + p] = lam0;
-        a.snap[2 * a.np + p] = ys0;
-        const float4 xm = __ldg(a.prev.x + p);
-        if (M.sel && __ldg(M.sel + p) != 0) {
-            // unsimulated: the G2P writes the reference's constant state, no P2G
-            a.cur.x[p] = make_float4(0.f, 0.f, 0.f, xm.w);
-            a.cur.v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            f9_store(a.cur.C, p, m3_zero());
-            f9_store(a.cur.F, p, m3_identity());
-        } else {
-            const float dt = L.steps[(size_t)g2p_table * L.n_inst + inst].dt;   // substep k-1
-            const V3 x = v3(xm.x, xm.y, xm.z);
-            const Stencil st = make_stencil(x, c.inv_dx);
-            const bool in_grid = stencil_in_grid(st, c.G);
-            const GlobalFetch fetch{vel, &c};
-            G2POut o;
-            if (MINB > 1) o = g2p_gather_rt(st, c.inv_dx, fetch.bind(st, in_grid));
-            else o = g2p_gather(st, c.inv_dx, fetch.bind(st, in_grid));
-            const float dx = 1.f / c.inv_dx;   // as g2p_particle computes it
-            const float lo = dx * 2.f, hi = c.grid_lim - dx * 2.f;
-            V3 nx = x + dt * o.v;
-            nx = v3(fminf(fmaxf(nx.x, lo), hi), fminf(fmaxf(nx.y, lo), hi), fminf(fmaxf(nx.z, lo), hi));
-            const M3 Fn = (m3_identity() + dt * o.gradv) * f9_load(a.fe_prev, p);
-            unsigned bad = 0;
-            if (!finite3(o.v) || !finite3(nx) || !isfinite(Fn.m[0] + Fn.m[4] + Fn.m[8])) bad |= EMPM_STATUS_NAN;
-            if (fmaxf(fmaxf(fabsf(o.v.x), fabsf(o.v.y)), fabsf(o.v.z)) * dt > dx) bad |= EMPM_STATUS_CFL;
-            if (!in_grid) bad |= EMPM_STATUS_OUT_OF_BAND;
-            if (bad) atomicOr(c.status, bad);
-            const EmpmStep& sp = *c.step;
-            V3 v = o.v;
-            if (sp.n_modifiers > 0) {
-                const int mi = M.pid ? __ldg(M.pid + p) : p;
-                apply_modifiers(sp, mi, nx, xm.w, v);
-            }
-            a.cur.x[p] = make_float4(nx.x, nx.y, nx.z, xm.w);
-            a.cur.v[p] = make_float4(v.x, v.y, v.z, 0.f);
-            f9_store(a.cur.C, p, o.C);
-            f9_store(a.cur.F, p, Fn);
-            float mu = mu0, lam = lam0, ys = ys0;
-            const ConstitutiveOut co = constitutive<MAT>(Fn, mu, lam, ys, sp.dt, *c.ms);
-            f9_store(a.fe_cur, p, co.F);
-            if (co.mat_changed) { M.mu[p] = mu; M.lam[p] = lam; M.ys[p] = ys; }
-            q.st = make_stencil(nx, c.inv_dx);
-            q.wm_scale = xm.w;
-            q.v = v;
-            q.Cd = damp_affine(o.C, c.rpic);
-            q.Sv = (-__ldg(M.vol + p)) * co.tau;
-            valid = true;
-        }
+    const bool valid = p < L.n_total && !(M.sel && __ldg(M.sel + p) != 0);
+    const float4 xm = p < L.n_total ? __ldg(a.prev.x + p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    V3 nx;
+    M3 Fn;
+    Ahead ah;
+    G2POut o;
+    if (valid) {
+        const float dt = L.steps[(size_t)g2p_table * L.n_inst + inst].dt;   // substep k-1
+        o = g2p_move(sh, c, dt, xm, a.fe_prev, M, p, vel, nx, Fn, ah);
+        a.snap[p] = ah.mu;
+        a.snap[a.np + p] = ah.lam;
+        a.snap[2 * a.np + p] = ah.ys;
+        a.cur.x[p] = make_float4(nx.x, nx.y, nx.z, xm.w);
+        f9_store(a.cur.C, p, o.C);
+        f9_store(a.cur.F, p, Fn);
+    } else if (p < L.n_total) {
+        // unsimulated: the G2P writes the reference's constant state, no P2G
+        a.snap[p] = __ldg(M.mu + p);
+        a.snap[a.np + p] = __ldg(M.lam + p);
+        a.snap[2 * a.np + p] = __ldg(M.ys + p);
+        a.cur.x[p] = make_float4(0.f, 0.f, 0.f, xm.w);
+        a.cur.v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        f9_store(a.cur.C, p, m3_zero());
+        f9_store(a.cur.F, p, m3_identity());
     }
-    warpagg_scatter<ROUNDS>(valid, inst, q, c, mom, flags);
+    p2g_cells<MAT>(sh, valid, c, *c.step, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, a.fe_cur,
+                   a.cur.v, mom, flags);
 }
 
-// k_g2p2g_store at the default run cap (4) for a launch whose instances all
-// use material (plasticine 5 and jelly 0 have kernels of their own, -1 any);
-// few: a launch over few particles (the MINB = 1 variant, as for k_g2p2g).
-// Returns false for other run caps (the caller runs the separate kernels).
-static inline bool launch_g2p2g_store(int grid_ctas, int threads, cudaStream_t s, const MaterialArrays& M,
-                                      const Launch& L, int g2p_table, const float4* vel, float4* mom,
-                                      unsigned char* flags, const SegmentStoreArgs& a, int seg_cap, int material,
-                                      bool few = false) {
-    if (seg_cap != 4) return false;
-    if (few && material == 5) k_g2p2g_store<2, 5, 1><<<grid_ctas, threads, 0, s>>>(M, L, g2p_table, vel, mom, flags, a);
-    else if (few && material == 0) k_g2p2g_store<2, 0, 1><<<grid_ctas, threads, 0, s>>>(M, L, g2p_table, vel, mom, flags, a);
-    else if (material == 5) k_g2p2g_store<2, 5><<<grid_ctas, threads, 0, s>>>(M, L, g2p_table, vel, mom, flags, a);
-    else if (material == 0) k_g2p2g_store<2, 0><<<grid_ctas, threads, 0, s>>>(M, L, g2p_table, vel, mom, flags, a);
-    else k_g2p2g_store<2, -1><<<grid_ctas, threads, 0, s>>>(M, L, g2p_table, vel, mom, flags, a);
-    return true;
+// Threads per CTA of the kernels above, and few: launches that would leave
+// SMs idle at the usual size (particle_threads) take the small CTAs.
+constexpr int kCellThreads = EMPM_CELL_THREADS;
+constexpr int kCellThreadsFew = 64;
+
+// One launch of a kernel template <NT, MAT, MINB>; material: the id every
+// instance of the launch uses (plasticine 5 and jelly 0 have kernels without
+// the other materials' code), or -1 when they differ.
+#define EMPM_CELL_LAUNCH(kernel, min_ctas, n, few, material, stream, ...)                                              \
+    do {                                                                                                             \
+        const int nt_ = (few) ? kCellThreadsFew : kCellThreads;                                                      \
+        const int g_ = ((n) + nt_ - 1) / nt_;                                                                        \
+        if (few) {                                                                                                   \
+            if ((material) == 5) kernel<kCellThreadsFew, 5, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                 \
+            else if ((material) == 0) kernel<kCellThreadsFew, 0, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);            \
+            else kernel<kCellThreadsFew, -1, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                                \
+        } else {                                                                                                     \
+            if ((material) == 5) kernel<kCellThreads, 5, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);             \
+            else if ((material) == 0) kernel<kCellThreads, 0, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);        \
+            else kernel<kCellThreads, -1, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                            \
+        }                                                                                                            \
+    } while (0)
+
+static inline void launch_g2p2g_store(bool few, cudaStream_t s, const MaterialArrays& M, const Launch& L,
+                                      int g2p_table, const float4* vel, float4* mom, unsigned char* flags,
+                                      const SegmentStoreArgs& a, int material) {
+    EMPM_CELL_LAUNCH(k_g2p2g_store, EMPM_FUSED_MIN_CTAS, L.n_total, few, material, s, M, L, g2p_table, vel, mom, flags, a);
 }
 
-static inline void launch_g2p2g(int grid_ctas, int threads, cudaStream_t s, const ParticleArrays& P,
-                                const MaterialArrays& M, const F9Planes& Fe, const Launch& L, int g2p_table,
-                                const float4* vel, float4* mom, unsigned char* flags, int seg_cap,
-                                int material = -1, bool few = false) {
-    // few: a launch over few particles (CTAs of 64 threads) takes the MINB = 1
-    // variant where one is compiled (plasticine and jelly at run cap 4)
-#define EMPM_G2P2G(R, MAT) k_g2p2g<R, MAT><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, g2p_table, vel, mom, flags)
-    if (few && material == 5 && seg_cap == 4) {
-        k_g2p2g<2, 5, 1><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, g2p_table, vel, mom, flags);
-        return;
-    }
-    if (few && material == 0 && seg_cap == 4) {
-        k_g2p2g<2, 0, 1><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, g2p_table, vel, mom, flags);
-        return;
-    }
-    if (material == 5 && seg_cap == 4) { EMPM_G2P2G(2, 5); return; }
-    if (material == 5 && seg_cap == 8) { EMPM_G2P2G(3, 5); return; }
-    if (material == 0 && seg_cap == 4) { EMPM_G2P2G(2, 0); return; }
-    if (material == 0 && seg_cap == 8) { EMPM_G2P2G(3, 0); return; }
-    switch (seg_cap) {
-        case 1: EMPM_G2P2G(0, -1); break;
-        case 2: EMPM_G2P2G(1, -1); break;
-        case 4: EMPM_G2P2G(2, -1); break;
-        case 8: EMPM_G2P2G(3, -1); break;
-        case 16: EMPM_G2P2G(4, -1); break;
-        default: EMPM_G2P2G(5, -1); break;
-    }
-#undef EMPM_G2P2G
+static inline void launch_g2p2g(bool few, cudaStream_t s, const ParticleArrays& P, const MaterialArrays& M,
+                                const F9Planes& Fe, const Launch& L, int g2p_table, const float4* vel, float4* mom,
+                                unsigned char* flags, int material) {
+    EMPM_CELL_LAUNCH(k_g2p2g, EMPM_FUSED_MIN_CTAS, L.n_total, few, material, s, P, M, Fe, L, g2p_table, vel, mom, flags);
 }
 
-// k_p2g_warpagg for a run cap seg_cap (a power of two in 1..32). material:
-// the material id every instance of the launch uses, or -1 when they differ;
-// plasticine (5) and jelly (0) at run caps 4 and 8 have kernels compiled for
-// that material alone.
-static inline void launch_p2g_warpagg(int grid_ctas, int threads, cudaStream_t s, const ParticleArrays& P,
-                                      const MaterialArrays& M, const F9Planes& Fe, const Launch& L, float4* mom,
-                                      unsigned char* flags, int seg_cap, int material = -1) {
-    if (material == 5 && seg_cap == 4) { k_p2g_warpagg<2, 5><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); return; }
-    if (material == 5 && seg_cap == 8) { k_p2g_warpagg<3, 5><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); return; }
-    if (material == 0 && seg_cap == 4) { k_p2g_warpagg<2, 0><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); return; }
-    if (material == 0 && seg_cap == 8) { k_p2g_warpagg<3, 0><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); return; }
-    switch (seg_cap) {
-        case 1: k_p2g_warpagg<0><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-        case 2: k_p2g_warpagg<1><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-        case 4: k_p2g_warpagg<2><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-        case 8: k_p2g_warpagg<3><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-        case 16: k_p2g_warpagg<4><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-        default: k_p2g_warpagg<5><<<grid_ctas, threads, 0, s>>>(P, M, Fe, L, mom, flags); break;
-    }
+static inline void launch_p2g_cells(bool few, cudaStream_t s, const ParticleArrays& P, const MaterialArrays& M,
+                                    const F9Planes& Fe, const Launch& L, float4* mom, unsigned char* flags,
+                                    int material) {
+    EMPM_CELL_LAUNCH(k_p2g_cells, EMPM_P2G_MIN_CTAS, L.n_total, few, material, s, P, M, Fe, L, mom, flags);
 }
 
 // -------------------------------------------------------------------------

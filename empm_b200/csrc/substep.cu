@@ -575,6 +575,8 @@ static int particle_threads(const EmpmCtx* ctx, long long n, int usual) {
     return blocks_for(n, usual) >= 2LL * ctx->sm_count ? usual : 64;
 }
 
+static bool few_particles(const EmpmCtx* ctx, long long n) { return particle_threads(ctx, n, 256) < 256; }
+
 // The material id all instances share, or -1 when they differ.
 static int uniform_material(const EmpmCtx* ctx) {
     if (ctx->n_inst < 1) return -1;
@@ -814,9 +816,8 @@ static int launch_p2g_sorted(EmpmCtx* ctx, const SortedState& ss, int table, cud
     const size_t smem = sizeof(float4) * (size_t)ctx->tile_cap;
     timing_mark(ctx, 0, 0, stream);
     if (ctx->p2g_mode == 2) {
-        const int tp = particle_threads(ctx, n, 256);
-        launch_p2g_warpagg(blocks_for(n, tp), tp, stream, t.P, t.M, t.Fe, t.L, ctx->grid_mom, ctx->flags,
-                           ctx->seg_cap, uniform_material(ctx));
+        launch_p2g_cells(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, ctx->grid_mom, ctx->flags,
+                         uniform_material(ctx));
     } else {
         k_p2g_tiled<<<ctx->sm_count * 2, TILE_THREADS, smem, stream>>>(t);
     }
@@ -856,10 +857,9 @@ static int launch_substep_sorted(EmpmCtx* ctx, SortedState& ss, int table, cudaS
 static int launch_g2p2g_sorted(EmpmCtx* ctx, const SortedState& ss, int g2p_table, int table, cudaStream_t stream) {
     const int n = ctx->n_particles;
     const TiledArgs t = sorted_args(ctx, ss, table);
-    const int tp = particle_threads(ctx, n, 256);
     timing_mark(ctx, 6, 0, stream);
-    launch_g2p2g(blocks_for(n, tp), tp, stream, t.P, t.M, t.Fe, t.L, g2p_table, ctx->grid_vel, ctx->grid_mom,
-                 ctx->flags, ctx->seg_cap, uniform_material(ctx), tp < 256);
+    launch_g2p2g(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, g2p_table, ctx->grid_vel, ctx->grid_mom,
+                 ctx->flags, uniform_material(ctx));
     timing_mark(ctx, 6, 1, stream);
     CK(cudaGetLastError(), "k_g2p2g");
     return EMPM_OK;
@@ -1381,8 +1381,8 @@ static int launch_substep_arrays(EmpmCtx* ctx, const ParticleArrays& Pin, const 
     const int n = ctx->n_particles;
     const Launch L = make_launch(ctx, table);
     timing_mark(ctx, 0, 0, s);
-    if (warpagg) launch_p2g_warpagg(blocks_for(n, 256), 256, s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags, ctx->seg_cap,
-                                    uniform_material(ctx));
+    if (warpagg) launch_p2g_cells(few_particles(ctx, n), s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags,
+                                  uniform_material(ctx));
     else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pin, M, Fe, L, ctx->grid_mom, ctx->flags);
     timing_mark(ctx, 0, 1, s);
     CK(cudaGetLastError(), "adjoint segment P2G");
@@ -1438,7 +1438,7 @@ static int segment_forward(EmpmCtx* ctx, const SegmentData& d, cudaStream_t s) {
     // sorted stored segments: from the second substep on, the G2P of the
     // previous substep and the stress + P2G of this one run as one kernel
     // that writes the stored state, snapshot and elastic F itself
-    const bool fused = d.store && d.sorted && ctx->fuse && ctx->seg_cap == 4 && d.n_steps > 1;
+    const bool fused = d.store && d.sorted && ctx->fuse && d.n_steps > 1;
     for (int k = 0; k < d.n_steps; ++k) {
         const ParticleArrays Pin = particle_arrays(d.states + (size_t)k * state_floats, n);
         const ParticleArrays Pout = particle_arrays(d.states + (size_t)(k + 1) * state_floats, n);
@@ -1460,17 +1460,16 @@ static int segment_forward(EmpmCtx* ctx, const SegmentData& d, cudaStream_t s) {
             sa.snap = d.mats + (size_t)k * 3 * np;
             sa.np = (long long)np;
             timing_mark(ctx, 6, 0, s);
-            const int tp = particle_threads(ctx, n, 256);
-            launch_g2p2g_store(blocks_for(n, tp), tp, s, Mw, Lk, k - 1, ctx->grid_vel, ctx->grid_mom, ctx->flags, sa,
-                               ctx->seg_cap, uniform_material(ctx), tp < 256);
+            launch_g2p2g_store(few_particles(ctx, n), s, Mw, Lk, k - 1, ctx->grid_vel, ctx->grid_mom, ctx->flags, sa,
+                               uniform_material(ctx));
             timing_mark(ctx, 6, 1, s);
             CK(cudaGetLastError(), "k_g2p2g_store");
         } else {
             CK(cudaMemcpyAsync(d.mats + (size_t)k * 3 * np, ab.work, 3 * np * sizeof(float), cudaMemcpyDeviceToDevice,
                                s), "snapshot");
             timing_mark(ctx, 0, 0, s);
-            if (d.sorted) launch_p2g_warpagg(blocks_for(n, 256), 256, s, Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags,
-                                             ctx->seg_cap, uniform_material(ctx));
+            if (d.sorted) launch_p2g_cells(few_particles(ctx, n), s, Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags,
+                                           uniform_material(ctx));
             else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags);
             timing_mark(ctx, 0, 1, s);
             CK(cudaGetLastError(), "adjoint segment P2G");
@@ -1535,8 +1534,8 @@ static int segment_reverse(EmpmCtx* ctx, const SegmentData& d, ParticleArrays Gp
                "restore snapshot");
             const Launch Lrec = make_launch_on(ctx, d.steps, n_steps + k);
             timing_mark(ctx, 0, 0, s);
-            if (d.sorted) launch_p2g_warpagg(blocks_for(n, 256), 256, s, Pk, Mw, Fe, Lrec, ctx->grid_mom,
-                                             ctx->flags, ctx->seg_cap, uniform_material(ctx));
+            if (d.sorted) launch_p2g_cells(few_particles(ctx, n), s, Pk, Mw, Fe, Lrec, ctx->grid_mom, ctx->flags,
+                                           uniform_material(ctx));
             else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pk, Mw, Fe, Lrec, ctx->grid_mom, ctx->flags);
             timing_mark(ctx, 0, 1, s);
             CK(cudaGetLastError(), "P2G (adjoint recompute)");

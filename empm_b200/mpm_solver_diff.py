@@ -115,10 +115,10 @@ class MPMWARPDiff(object):
         self.use_graph = True
         # launch options of the library (see EMPM_OPT_* in include/empm_b200.h)
         self.sort_every = 32
-        self.p2g_mode = 2          # 0 direct, 1 shared-memory tile, 2 warp-aggregated
+        self.p2g_mode = 2          # 0 direct, 1 shared-memory tile, 2 summed per cell
         self.g2p_tile = False
         self.tile_cap = 1024
-        self.seg_cap = 4           # warp-aggregated P2G: longest same-cell run per reduction
+        self.seg_cap = 4           # G2P adjoint: longest same-cell run per reduction
         self.adj_store = True      # adjoint keeps each substep's grid and elastic F instead of recomputing
         self.fuse = True           # rollouts fuse each G2P with the next substep's stress + P2G
         self.segment_graph = True  # stored tape segments replay their substep loops from CUDA graphs

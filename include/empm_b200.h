@@ -301,19 +301,19 @@ int  empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const Emp
 /* Launch options of a context (empm_ctx_set_option). */
 #define EMPM_OPT_SORT_EVERY  1   /* rollouts re-sort particles by 4^3 cell block every N substeps; 0 = no sorting (default 32) */
 #define EMPM_OPT_P2G_MODE    2   /* sorted-path P2G: 0 = one 16-byte reduction per particle and node,
-                                    1 = shared-memory node tile per chunk, 2 = warp-aggregated reductions
-                                    over same-cell particles (default) */
+                                    1 = shared-memory node tile per chunk, 2 = contributions summed per cell
+                                    in shared memory (default) */
 #define EMPM_OPT_G2P_TILE    3   /* 1 = G2P stages the node tile in shared memory (default), 0 = direct gathers */
 #define EMPM_OPT_TILE_CAP    4   /* nodes per shared-memory tile, 27..3072 (default 1024 = 16 KiB) */
-#define EMPM_OPT_SEG_CAP     5   /* warp-aggregated P2G: same-cell runs longer than this (a power of two,
-                                    1..32 lanes) are split, trading shuffle rounds for grid reductions
-                                    (default 4) */
+#define EMPM_OPT_SEG_CAP     5   /* G2P adjoint: same-cell runs longer than this (a power of two, 1..32
+                                    lanes) are split, trading shuffle rounds for grid reductions
+                                    (default 4); the P2G kernels sum whole cells */
 #define EMPM_OPT_ADJ_STORE   6   /* empm_adjoint_segment: 1 = keep every substep's touched grid blocks and
                                     elastic F from the segment's forward pass for the reverse pass (default;
                                     n_steps x (2 KiB per grid block + 36 B per particle) of device memory,
                                     recompute when that allocation fails); 0 = recompute P2G and the grid
                                     update in the reverse pass */
-#define EMPM_OPT_FUSE        7   /* sorted rollouts with warp-aggregated P2G and direct G2P: 1 = between two cell
+#define EMPM_OPT_FUSE        7   /* sorted rollouts with P2G mode 2 and direct G2P: 1 = between two cell
                                     sorts, the G2P of each substep and the stress + P2G of the next run as one
                                     kernel that keeps only position and elastic F per particle between substeps
                                     (default); 0 = separate kernels. Step tables that release a held instance
