@@ -143,6 +143,8 @@ def lib():
         "empm_debug_stress_adjoint": ([ctypes.POINTER(EmpmModelParams), P, P, P, P, ctypes.c_float, P, P, P, P, P,
                                        P, I, P], I),
         "empm_knn": ([P, I, P, I, I, I, P, I, P, P], I),
+        "empm_knn_workspace": ([I, I, I, ctypes.POINTER(ctypes.c_size_t)], I),
+        "empm_knn_cells": ([P, I, P, I, I, I, P, I, P, P, ctypes.c_size_t, P], I),
         "empm_idw_weights": ([P, I, P, I, P, I, I, P, P, P], I),
         "empm_lbs_bones": ([P, P, I, P, I, I, I, P, P, P, P], I),
         "empm_lbs_blend": ([P, I, P, P, I, P, I, I, P, P, P, P, P, P], I),

@@ -133,74 +133,37 @@ __device__ __forceinline__ float4 qmul(float4 a, float4 b) {
 }
 
 // ---------------------------------------------------------------------------
-// k nearest neighbours: one query per thread, candidates staged through
-// shared memory, the KT best kept sorted in registers
-// ---------------------------------------------------------------------------
-constexpr int kKnnThreads = 128;
-constexpr int kKnnTile = 1024;
-
-template <int KT, typename IdxT>
-__global__ void __launch_bounds__(kKnnThreads) k_knn(const float* __restrict__ q, int nq, const float* __restrict__ pts,
-                                                     int np, int k, int exclude_self, IdxT* __restrict__ out_idx,
-                                                     float* __restrict__ out_dist) {
-    __shared__ float4 tile[kKnnTile];
-    const int i = blockIdx.x * kKnnThreads + threadIdx.x;
-    const bool live = i < nq;
-    float qx = 0.f, qy = 0.f, qz = 0.f;
-    if (live) { qx = __ldg(q + 3 * (long long)i); qy = __ldg(q + 3 * (long long)i + 1); qz = __ldg(q + 3 * (long long)i + 2); }
-    float bd[KT];
-    int bi[KT];
-#pragma unroll
-    for (int s = 0; s < KT; ++s) { bd[s] = INFINITY; bi[s] = -1; }
-    const int self = (live && exclude_self) ? i : -1;
-    for (int base = 0; base < np; base += kKnnTile) {
-        const int m = min(kKnnTile, np - base);
-        __syncthreads();
-        for (int t = threadIdx.x; t < m; t += kKnnThreads) {
-            const long long j = base + t;
-            tile[t] = make_float4(__ldg(pts + 3 * j), __ldg(pts + 3 * j + 1), __ldg(pts + 3 * j + 2), 0.f);
-        }
-        __syncthreads();
-        for (int t = 0; t < m; ++t) {
-            const float4 p = tile[t];
-            const float dx = qx - p.x, dy = qy - p.y, dz = qz - p.z;
-            const float d = dx * dx + dy * dy + dz * dz;
-            const int j = base + t;
-            if (d < bd[KT - 1] && j != self) {
-                // insertion keeps equal distances in index order (strict <)
-#pragma unroll
-                for (int s = KT - 1; s > 0; --s) {
-                    if (d < bd[s - 1]) { bd[s] = bd[s - 1]; bi[s] = bi[s - 1]; }
-                    else if (d < bd[s]) { bd[s] = d; bi[s] = j; }
-                }
-                if (d < bd[0]) { bd[0] = d; bi[0] = j; }
-            }
-        }
-    }
-    if (!live) return;
-#pragma unroll
-    for (int s = 0; s < KT; ++s) {
-        if (s < k) {
-            out_idx[(long long)i * k + s] = (IdxT)bi[s];
-            if (out_dist) out_dist[(long long)i * k + s] = sqrtf(bd[s]);
-        }
-    }
-}
-
-template <typename IdxT>
-int launch_knn(const float* q, int nq, const float* pts, int np, int k, int exclude_self, IdxT* idx, float* dist,
-               cudaStream_t s) {
-    const int g = blocks_for(nq, kKnnThreads);
-    if (k <= 8) k_knn<8, IdxT><<<g, kKnnThreads, 0, s>>>(q, nq, pts, np, k, exclude_self, idx, dist);
-    else if (k <= 16) k_knn<16, IdxT><<<g, kKnnThreads, 0, s>>>(q, nq, pts, np, k, exclude_self, idx, dist);
-    else k_knn<32, IdxT><<<g, kKnnThreads, 0, s>>>(q, nq, pts, np, k, exclude_self, idx, dist);
-    CKB(cudaGetLastError(), "k_knn");
-    return EMPM_OK;
-}
-
-// ---------------------------------------------------------------------------
 // inverse-distance weights of k given bones (calc_weights_vals_from_indices)
 // ---------------------------------------------------------------------------
+// One thread per (point, bone) pair, W (a power of two >= k) neighbouring lanes per
+// point: the index rows and weights are read and written coalesced, where a thread
+// per point touched a sector per index (500k points, k = 16, 8-byte indices: 191 ->
+// 69 us; what is left are the 16 unrelated bone positions of every point).
+template <int W, typename IdxT>
+__global__ void __launch_bounds__(256) k_idw_lanes(const float* __restrict__ bones, int n_bones,
+                                                   const float* __restrict__ pts, int n,
+                                                   const IdxT* __restrict__ idx, int k, float* __restrict__ w,
+                                                   int* __restrict__ status) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long p = t / W;
+    const int s = (int)(t % W);
+    const bool on = p < n && s < k;
+    float v = 0.f;
+    bool bad = false;
+    if (on) {
+        const long long b = load_idx(idx, p * k + s);
+        bad = b < 0 || b >= n_bones;
+        if (!bad) v = 1.f / (length(load3(pts, p) - load3(bones, b)) + 1e-6f);
+    }
+    // in index order, as the blend sums them: the weights are the same to the bit
+    float sum = 0.f;
+    for (int e = 0; e < k; ++e) sum += __shfl_sync(0xffffffffu, v, e, W);
+    const unsigned bads = __ballot_sync(0xffffffffu, bad);
+    const unsigned mine = (W == 32 ? 0xffffffffu : ((1u << W) - 1u)) << ((threadIdx.x & 31) & ~(W - 1));
+    if (on) w[p * k + s] = bads & mine ? __int_as_float(0x7fc00000) : v / sum;
+    if (bads && (threadIdx.x & 31) == 0) atomicOr(status, kBadIndex);
+}
+
 template <typename IdxT>
 __global__ void k_idw(const float* __restrict__ bones, int n_bones, const float* __restrict__ pts, int n,
                       const IdxT* __restrict__ idx, int k, float* __restrict__ w, int* __restrict__ status) {
@@ -222,6 +185,17 @@ __global__ void k_idw(const float* __restrict__ bones, int n_bones, const float*
         w[(long long)p * k + s] = v;
     }
     if (bad) atomicOr(status, kBadIndex);
+}
+
+template <typename IdxT>
+void launch_idw(const float* bones, int n_bones, const float* pts, int n, const IdxT* idx, int k, float* w, int* status,
+                cudaStream_t s) {
+    const auto g = [&](int width) { return blocks_for((long long)n * width, 256); };
+    if (k > 32) k_idw<<<blocks_for(n, 256), 256, 0, s>>>(bones, n_bones, pts, n, idx, k, w, status);
+    else if (k > 16) k_idw_lanes<32><<<g(32), 256, 0, s>>>(bones, n_bones, pts, n, idx, k, w, status);
+    else if (k > 8) k_idw_lanes<16><<<g(16), 256, 0, s>>>(bones, n_bones, pts, n, idx, k, w, status);
+    else if (k > 4) k_idw_lanes<8><<<g(8), 256, 0, s>>>(bones, n_bones, pts, n, idx, k, w, status);
+    else k_idw_lanes<4><<<g(4), 256, 0, s>>>(bones, n_bones, pts, n, idx, k, w, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -644,23 +618,6 @@ bool idx_ok(int idx_bytes) { return idx_bytes == 4 || idx_bytes == 8; }
 
 }  // namespace
 
-extern "C" int empm_knn(const float* queries, int n_queries, const float* points, int n_points, int k,
-                        int exclude_self, void* out_idx, int idx_bytes, float* out_dist, void* stream) {
-    if (n_queries < 0 || n_points < 0 || k < 1 || k > EMPM_KNN_MAX_K || !idx_ok(idx_bytes))
-        return empm_set_error(nullptr, EMPM_ERR_INVALID, "knn: bad sizes (k %d, idx_bytes %d)", k, idx_bytes);
-    if (exclude_self && n_queries != n_points)
-        return empm_set_error(nullptr, EMPM_ERR_INVALID, "knn: exclude_self needs queries == points");
-    if (k > n_points - (exclude_self ? 1 : 0))
-        return empm_set_error(nullptr, EMPM_ERR_INVALID, "knn: k %d exceeds the %d candidates", k,
-                              n_points - (exclude_self ? 1 : 0));
-    if (n_queries == 0) return EMPM_OK;
-    if (!queries || !points || !out_idx) return empm_set_error(nullptr, EMPM_ERR_INVALID, "knn: NULL pointer");
-    cudaStream_t s = (cudaStream_t)stream;
-    if (idx_bytes == 8)
-        return launch_knn(queries, n_queries, points, n_points, k, exclude_self, (long long*)out_idx, out_dist, s);
-    return launch_knn(queries, n_queries, points, n_points, k, exclude_self, (int*)out_idx, out_dist, s);
-}
-
 extern "C" int empm_idw_weights(const float* bones, int n_bones, const float* pts, int n, const void* idx,
                                 int idx_bytes, int k, float* weights, int* status, void* stream) {
     if (n < 0 || n_bones < 0 || k < 1 || !idx_ok(idx_bytes))
@@ -669,10 +626,8 @@ extern "C" int empm_idw_weights(const float* bones, int n_bones, const float* pt
     if (!bones || !pts || !idx || !weights || !status)
         return empm_set_error(nullptr, EMPM_ERR_INVALID, "idw weights: NULL pointer");
     cudaStream_t s = (cudaStream_t)stream;
-    if (idx_bytes == 8)
-        k_idw<<<blocks_for(n, 256), 256, 0, s>>>(bones, n_bones, pts, n, (const long long*)idx, k, weights, status);
-    else
-        k_idw<<<blocks_for(n, 256), 256, 0, s>>>(bones, n_bones, pts, n, (const int*)idx, k, weights, status);
+    if (idx_bytes == 8) launch_idw(bones, n_bones, pts, n, (const long long*)idx, k, weights, status, s);
+    else launch_idw(bones, n_bones, pts, n, (const int*)idx, k, weights, status, s);
     CKB(cudaGetLastError(), "k_idw");
     return EMPM_OK;
 }

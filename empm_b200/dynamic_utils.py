@@ -23,6 +23,7 @@ Differences from the reference, by design:
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Tuple
 
 import torch
@@ -103,11 +104,14 @@ def rotation_matrix_to_quaternion(rotation_matrix: Tensor) -> Tensor:
 # ---------------------------------------------------------------------------
 def _knn(queries: Tensor, points: Tensor, k: int, exclude_self: bool) -> Tuple[Tensor, Tensor]:
     q = _f32(queries, "queries", 3)
-    p = _f32(points, "points", 3)
+    p = q if exclude_self else _f32(points, "points", 3)   # the points themselves
     idx = torch.empty(q.shape[0], k, dtype=torch.int64, device=q.device)
     dist = torch.empty(q.shape[0], k, dtype=torch.float32, device=q.device)
-    N.check(N.lib().empm_knn(q.data_ptr(), q.shape[0], p.data_ptr(), p.shape[0], int(k), int(exclude_self),
-                             idx.data_ptr(), 8, dist.data_ptr(), _stream(q)))
+    nb = ctypes.c_size_t()
+    N.check(N.lib().empm_knn_workspace(q.shape[0], p.shape[0], int(exclude_self), ctypes.byref(nb)))
+    work = torch.empty(nb.value, dtype=torch.uint8, device=q.device)   # 512-byte aligned, as every torch block
+    N.check(N.lib().empm_knn_cells(q.data_ptr(), q.shape[0], p.data_ptr(), p.shape[0], int(k), int(exclude_self),
+                                   idx.data_ptr(), 8, dist.data_ptr(), work.data_ptr(), nb.value, _stream(q)))
     return idx, dist
 
 

@@ -519,6 +519,14 @@ int  empm_chamfer_backward(const float* x, const int* x_off, int nx, const float
 int  empm_knn(const float* queries, int n_queries, const float* points, int n_points, int k, int exclude_self,
               void* out_idx, int idx_bytes, float* out_dist, void* stream);
 
+/* The same results from a search in a cell grid, which sorts points and queries
+ * into a caller's device workspace of empm_knn_workspace bytes (256-byte
+ * aligned; 0 bytes: the sets are small and searched by brute force). */
+int  empm_knn_workspace(int n_queries, int n_points, int exclude_self, size_t* bytes);
+int  empm_knn_cells(const float* queries, int n_queries, const float* points, int n_points, int k, int exclude_self,
+                    void* out_idx, int idx_bytes, float* out_dist, void* workspace, size_t workspace_bytes,
+                    void* stream);
+
 /* Inverse-distance weights of the k given bones of every point:
  * w = 1 / (|x - b| + 1e-6), normalised over the k
  * (calc_weights_vals_from_indices, dynamic_utils.py:282-292). */

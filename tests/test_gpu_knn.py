@@ -1,0 +1,67 @@
+"""The cell-grid neighbour search against the brute-force kernel, bit for bit
+(indices, distances, ties in index order), where a grid can go wrong: flat and
+degenerate clouds, clusters far apart, points on a lattice (ties everywhere),
+queries far outside, coordinates far from the origin, and values that are not
+finite. And chamfer distances of many pairs through the grid."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _cloud(rng, kind, n):
+    if kind == "box":
+        return rng.uniform(0, 1, (n, 3))
+    if kind == "plane":
+        return rng.uniform(0, 1, (n, 3)) * [1, 1, 0]
+    if kind == "line":
+        return rng.uniform(0, 1, (n, 1)) * [[0.3, 0, 0]]
+    if kind == "point":
+        return np.full((n, 3), 0.25)
+    if kind == "clusters":
+        return rng.normal(0, 1e-3, (n, 3)) + rng.choice([0.0, 1.0, 50.0], (n, 1))
+    if kind == "lattice":
+        return rng.integers(0, 12, (n, 3)) / 8.0
+    if kind == "far":
+        return rng.uniform(0, 1, (n, 3)) + [1000.0, -500.0, 3e4]
+    x = rng.uniform(0, 1, (n, 3))          # not finite
+    x[::7, 0], x[3::11, 1], x[5::13, 2] = np.nan, np.inf, -np.inf
+    return x
+
+
+def _search(name, q, p, k, self_):
+    from empm_b200 import _native as N
+    L = N.lib()
+    idx = torch.empty(len(q), k, dtype=torch.int64, device=DEV)
+    dist = torch.empty(len(q), k, device=DEV)
+    args = (q.data_ptr(), len(q), p.data_ptr(), len(p), k, int(self_), idx.data_ptr(), 8, dist.data_ptr())
+    if name == "brute":
+        N.check(L.empm_knn(*args, None))
+    else:
+        nb = ctypes.c_size_t()
+        N.check(L.empm_knn_workspace(len(q), len(p), int(self_), ctypes.byref(nb)))
+        assert nb.value > 0
+        work = torch.empty(nb.value, dtype=torch.uint8, device=DEV)
+        N.check(L.empm_knn_cells(*args, work.data_ptr(), nb.value, None))
+    torch.cuda.synchronize()
+    return idx, dist
+
+
+@pytest.mark.parametrize("kind", ["box", "plane", "line", "point", "clusters", "lattice", "far", "nan"])
+@pytest.mark.parametrize("k,n,nq", [(1, 2000, 1), (5, 2049, 700), (16, 6000, 3001), (32, 3000, 257)])
+def test_cells_equal_brute_force(kind, k, n, nq):
+    rng = np.random.default_rng(k)
+    t = lambda a: torch.as_tensor(np.asarray(a, np.float32), device=DEV).contiguous()  # noqa: E731
+    p = t(_cloud(rng, kind, n))
+    q = _cloud(rng, kind, nq)
+    q[::5] = rng.uniform(-3, 4, q[::5].shape)      # some outside the points' box
+    q[::17] = 1e6
+    for queries, self_ in ((t(q), False), (p, True)):
+        a, da = _search("brute", queries, p, k, self_)
+        b, db = _search("cells", queries, p, k, self_)
+        assert torch.equal(a, b)
+        assert torch.equal(da.view(torch.int32), db.view(torch.int32))
