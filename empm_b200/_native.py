@@ -138,6 +138,8 @@ def lib():
                                   ctypes.POINTER(EmpmParticles), P], I),
         "empm_segment_reverse": ([P, P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmMaterialGrad), P], I),
         "empm_chamfer": ([P, P, I, I, P, P, I, I, I, P, P, P, P, P], I),
+        "empm_chamfer_workspace": ([I, I, I, I, I, ctypes.POINTER(ctypes.c_size_t)], I),
+        "empm_chamfer_cells": ([P, P, I, I, P, P, I, I, I, P, P, P, P, P, ctypes.c_size_t, P], I),
         "empm_restart_F": ([P, ctypes.POINTER(EmpmParticles), P, P, P, P], I),
         "empm_chamfer_backward": ([P, P, I, P, P, I, I, P, P, P, P, P, P, P], I),
         "empm_debug_stress_adjoint": ([ctypes.POINTER(EmpmModelParams), P, P, P, P, ctypes.c_float, P, P, P, P, P,

@@ -79,14 +79,14 @@ __device__ __forceinline__ float float_decode(unsigned u) {
     return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
 }
 
-__global__ void k_box_init(unsigned* box, int n6) {
+static __global__ void k_box_init(unsigned* box, int n6) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n6) box[i] = (i % 6) < 3 ? 0xffffffffu : 0u;
 }
 
 // Bounding boxes of the finite points, 512 points per warp: one set of atomics
 // per warp and set (two of a million points, 2 k of them, meet on a word).
-__global__ void __launch_bounds__(256) k_box(const PointSets P, int n, unsigned* box) {
+static __global__ void __launch_bounds__(256) k_box(const PointSets P, int n, unsigned* box) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     unsigned v[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     int cur = -1;   // the set the accumulated box belongs to (the same in every lane)
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) k_box(const PointSets P, int n, unsigned*
 
 // Grid of each set: cubic cells with about `per_cell` points, axes thinner than a
 // cell left whole. share: set 1 uses set 0's grid (queries binned like the points).
-__global__ void k_grid_setup(const PointSets P, const unsigned* box, SetGrid* grids, float per_cell, int share) {
+static __global__ void k_grid_setup(const PointSets P, const unsigned* box, SetGrid* grids, float per_cell, int share) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= P.sets()) return;
     const bool in_a = s < P.sets_a;
@@ -196,7 +196,7 @@ __device__ __forceinline__ int cell_bin(const SetGrid& g, float x, float y, floa
 }
 
 // start[c + 1] counts bin c
-__global__ void __launch_bounds__(256) k_bin_count(const PointSets P, int n, const SetGrid* grids, int* start) {
+static __global__ void __launch_bounds__(256) k_bin_count(const PointSets P, int n, const SetGrid* grids, int* start) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float x, y, z;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256) k_bin_count(const PointSets P, int n, con
 
 constexpr int kScanTile = 2048;
 
-__global__ void __launch_bounds__(256) k_scan_sums(const int* v, int n, int* sums) {
+static __global__ void __launch_bounds__(256) k_scan_sums(const int* v, int n, int* sums) {
     __shared__ int part[8];
     const int t = threadIdx.x;
     int s = 0;
@@ -248,7 +248,7 @@ __device__ __forceinline__ int block_scan(int v, int* part, int& total) {
     return before + incl - v;
 }
 
-__global__ void __launch_bounds__(256) k_scan_top(int* sums, int n) {
+static __global__ void __launch_bounds__(256) k_scan_top(int* sums, int n) {
     __shared__ int part[8];
     int carry = 0;
     for (int b = 0; b < n; b += 256) {
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) k_scan_top(int* sums, int n) {
 }
 
 // v[i] <- exclusive sum
-__global__ void __launch_bounds__(256) k_scan_apply(int* v, int n, const int* sums) {
+static __global__ void __launch_bounds__(256) k_scan_apply(int* v, int n, const int* sums) {
     __shared__ int part[8];
     const int i0 = blockIdx.x * kScanTile + threadIdx.x * 8;
     int e[8], s = 0;
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) k_scan_apply(int* v, int n, const int* su
 
 // Points to their bins: (x, y, z, row). Afterwards bin c holds
 // sorted[start[c] .. start[c + 1]) (start[0] is 0).
-__global__ void __launch_bounds__(256) k_bin_scatter(const PointSets P, int n, const SetGrid* grids, int* start,
+static __global__ void __launch_bounds__(256) k_bin_scatter(const PointSets P, int n, const SetGrid* grids, int* start,
                                                      float4* sorted) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

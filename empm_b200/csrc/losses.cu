@@ -7,12 +7,17 @@
 // min_x |x - y|^2 (point_reduction "mean"). Here many (X, Y) pairs (one per
 // population member and frame) are scored in one launch: pair p owns
 // X rows [x_off[p], x_off[p+1]) and Y rows [y_off[p], y_off[p+1]). The nearest
-// neighbours are found exactly, by brute force over shared-memory tiles of
-// the other set, and kept for the gradient.
+// neighbours are found exactly, in cell grids of the clouds (cellgrid.cuh) or, for
+// small ones, by brute force over shared-memory tiles of the other set, with the
+// same results, and kept for the gradient.
 #include <cuda_runtime.h>
 #include <float.h>
+#include <stdint.h>
 #include "../../include/empm_b200.h"
+#include "cellgrid.cuh"
 #include "ctx.hpp"
+
+using namespace empm;
 
 namespace {
 
@@ -45,8 +50,7 @@ __global__ void __launch_bounds__(kThreads) k_nn(const float* __restrict__ q, co
         const int m = min(kThreads, t1 - base);
         for (int k = 0; k < m; ++k) {
             const float4 p = tile[k];
-            const float dx = qx - p.x, dy = qy - p.y, dz = qz - p.z;
-            const float d = dx * dx + dy * dy + dz * dz;
+            const float d = point_dist2(qx, qy, qz, p.x, p.y, p.z);
             if (d < best) { best = d; arg = base + k; }
         }
     }
@@ -56,6 +60,49 @@ __global__ void __launch_bounds__(kThreads) k_nn(const float* __restrict__ q, co
     float v = (live && arg >= 0) ? best : 0.f;
     for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
     if ((threadIdx.x & 31) == 0 && v != 0.f) atomicAdd(sum + pair, v);
+}
+
+// The same through cell grids: one thread per point of either cloud, in the order
+// of its own cloud's cells, searching the other cloud of its pair. Clouds of the
+// same size apart, the 27 cells around a query hold about 54 candidates.
+__global__ void __launch_bounds__(kThreads) k_nn_cells(const PointSets P, const CellGridWork w,
+                                                       int* __restrict__ nn_x, int* __restrict__ nn_y,
+                                                       float* __restrict__ sum_xy, float* __restrict__ sum_yx) {
+    __shared__ float part[kThreads / 32];
+    __shared__ int ends[2];
+    const int t = blockIdx.x * kThreads + threadIdx.x;
+    const int n = P.rows();
+    float v = 0.f;
+    int set = -1;
+    if (t < n) {
+        const bool in_a = t < P.rows_a;
+        const int pair = in_a ? set_find(P.a_off, P.sets_a, t) : set_find(P.b_off, P.sets_b, t - P.rows_a);
+        set = in_a ? pair : P.sets_a + pair;
+        const float4 q = __ldg(w.sorted + t);
+        Nearest<1> best;
+        best.clear(FLT_MAX);
+        nearest_search<1>(w.grids[in_a ? P.sets_a + pair : pair], w.start, w.sorted, q.x, q.y, q.z, 1, -1, 1, best);
+        (in_a ? nn_x : nn_y)[__float_as_int(q.w)] = best.i[0];
+        if (best.i[0] >= 0) v = best.d[0];
+    }
+    // one atomic per block, or per thread where two clouds meet in it
+    if (threadIdx.x == 0) ends[0] = set;
+    if (threadIdx.x == min(kThreads, n - (int)(blockIdx.x * kThreads)) - 1) ends[1] = set;
+    __syncthreads();
+    float* sum = set < 0 ? nullptr : (set < P.sets_a ? sum_xy + set : sum_yx + (set - P.sets_a));
+    if (ends[0] != ends[1]) {
+        if (v != 0.f) atomicAdd(sum, v);
+        return;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float s = 0.f;
+        for (int k = 0; k < kThreads / 32; ++k) s += part[k];
+        if (s != 0.f) atomicAdd(sum, s);
+    }
 }
 
 // Gradient in X of  g_xy[p] * sum_i |x_i - y_nn(i)|^2 + g_yx[p] * sum_j |y_j - x_nn(j)|^2
@@ -104,13 +151,58 @@ __global__ void k_pair_index(const int* off, int n_pairs, int* pair_of, int n) {
         if (_rc != EMPM_OK) return _rc;                                          \
     } while (0)
 
-extern "C" int empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,
-                            int ny, int max_ny, int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y,
-                            void* stream) {
+static int check_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off, int ny,
+                         int max_ny, int n_pairs, const float* sum_xy, const float* sum_yx, const int* nn_x,
+                         const int* nn_y) {
     if (n_pairs < 1 || n_pairs > 65535 || nx < 0 || ny < 0 || max_nx < 0 || max_ny < 0)
         return empm_set_error(nullptr, EMPM_ERR_INVALID, "bad chamfer sizes (%d pairs)", n_pairs);
     if (!x_off || !y_off || !sum_xy || !sum_yx || (nx && (!x || !nn_x)) || (ny && (!y || !nn_y)))
         return empm_set_error(nullptr, EMPM_ERR_INVALID, "chamfer pointer is NULL");
+    return EMPM_OK;
+}
+
+extern "C" int empm_chamfer_workspace(int nx, int max_nx, int ny, int max_ny, int n_pairs, size_t* bytes) {
+    if (n_pairs < 1 || nx < 0 || ny < 0 || max_nx < 0 || max_ny < 0 || !bytes)
+        return empm_set_error(nullptr, EMPM_ERR_INVALID, "bad chamfer sizes (%d pairs)", n_pairs);
+    // The brute-force search looks at 2.2e12 pairs of points a second; the grids'
+    // ten launches and the sorting take about 60 us before the search, as long as
+    // 7e7 pairs in each direction.
+    *bytes = 0;
+    if ((double)n_pairs * max_nx * max_ny < 7e7 || (long long)nx + ny > (1LL << 30)) return EMPM_OK;
+    const PointSets P{nullptr, nullptr, n_pairs, nx, nullptr, nullptr, n_pairs, ny};
+    *bytes = cellgrid_layout(P, 0, nullptr, nullptr);
+    return EMPM_OK;
+}
+
+extern "C" int empm_chamfer_cells(const float* x, const int* x_off, int nx, int max_nx, const float* y,
+                                  const int* y_off, int ny, int max_ny, int n_pairs, float* sum_xy, float* sum_yx,
+                                  int* nn_x, int* nn_y, void* workspace, size_t workspace_bytes, void* stream) {
+    const int rc = check_chamfer(x, x_off, nx, max_nx, y, y_off, ny, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y);
+    if (rc) return rc;
+    size_t need = 0;
+    empm_chamfer_workspace(nx, max_nx, ny, max_ny, n_pairs, &need);
+    if (need == 0)
+        return empm_chamfer(x, x_off, nx, max_nx, y, y_off, ny, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y, stream);
+    if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255))
+        return empm_set_error(nullptr, EMPM_ERR_INVALID, "chamfer: workspace of %zu bytes, 256-byte aligned, needed",
+                              need);
+    cudaStream_t s = (cudaStream_t)stream;
+    CKL(cudaMemsetAsync(sum_xy, 0, sizeof(float) * n_pairs, s), "chamfer");
+    CKL(cudaMemsetAsync(sum_yx, 0, sizeof(float) * n_pairs, s), "chamfer");
+    const PointSets P{x, x_off, n_pairs, nx, y, y_off, n_pairs, ny};
+    CellGridWork w;
+    cellgrid_layout(P, 0, workspace, &w);
+    CKL(cellgrid_build(P, 0, 2.f, w, s), "chamfer cell grids");
+    k_nn_cells<<<blocks_for((long long)nx + ny, kThreads), kThreads, 0, s>>>(P, w, nn_x, nn_y, sum_xy, sum_yx);
+    CKL(cudaGetLastError(), "k_nn_cells");
+    return EMPM_OK;
+}
+
+extern "C" int empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,
+                            int ny, int max_ny, int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y,
+                            void* stream) {
+    const int rc = check_chamfer(x, x_off, nx, max_nx, y, y_off, ny, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y);
+    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     CKL(cudaMemsetAsync(sum_xy, 0, sizeof(float) * n_pairs, s), "chamfer");
     CKL(cudaMemsetAsync(sum_yx, 0, sizeof(float) * n_pairs, s), "chamfer");

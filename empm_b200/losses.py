@@ -12,6 +12,7 @@
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional, Sequence, Tuple
 
 import numpy as np
@@ -40,9 +41,13 @@ class _ChamferPairs(torch.autograd.Function):
         s_yx = torch.empty_like(s_xy)
         nn_x = torch.empty(x.shape[0], dtype=torch.int32, device=dev)
         nn_y = torch.empty(y.shape[0], dtype=torch.int32, device=dev)
-        N.check(N.lib().empm_chamfer(x.data_ptr(), x_off.data_ptr(), x.shape[0], max_nx, y.data_ptr(),
-                                     y_off.data_ptr(), y.shape[0], max_ny, n_pairs, s_xy.data_ptr(), s_yx.data_ptr(),
-                                     nn_x.data_ptr(), nn_y.data_ptr(), _stream_ptr(dev)))
+        nb = ctypes.c_size_t()
+        N.check(N.lib().empm_chamfer_workspace(x.shape[0], max_nx, y.shape[0], max_ny, n_pairs, ctypes.byref(nb)))
+        work = torch.empty(nb.value, dtype=torch.uint8, device=dev)   # 512-byte aligned, as every torch block
+        N.check(N.lib().empm_chamfer_cells(x.data_ptr(), x_off.data_ptr(), x.shape[0], max_nx, y.data_ptr(),
+                                           y_off.data_ptr(), y.shape[0], max_ny, n_pairs, s_xy.data_ptr(),
+                                           s_yx.data_ptr(), nn_x.data_ptr(), nn_y.data_ptr(), work.data_ptr(),
+                                           nb.value, _stream_ptr(dev)))
         nx = torch.as_tensor(np.maximum(np.asarray(x_counts), 1), dtype=torch.float32, device=dev)
         ny = torch.as_tensor(np.maximum(np.asarray(y_counts), 1), dtype=torch.float32, device=dev)
         ctx.save_for_backward(x, y, x_off, y_off, nn_x, nn_y, nx, ny)

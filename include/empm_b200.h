@@ -488,6 +488,15 @@ int  empm_restart_F(EmpmCtx* ctx, EmpmParticles* particles, const float* target,
 int  empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off, int ny,
                   int max_ny, int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y, void* stream);
 
+/* The same through cell grids of the clouds, in a caller's device workspace of
+ * empm_chamfer_workspace bytes (256-byte aligned; 0 bytes: the clouds are small and
+ * searched by brute force). Neighbours are the same; the sums differ by the order
+ * of their single-precision additions. */
+int  empm_chamfer_workspace(int nx, int max_nx, int ny, int max_ny, int n_pairs, size_t* bytes);
+int  empm_chamfer_cells(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,
+                        int ny, int max_ny, int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y,
+                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* Gradient in x of sum_p (g_xy[p] * sum_xy[p] + g_yx[p] * sum_yx[p]) for the
  * neighbours found by empm_chamfer, ADDED to grad_x ([nx, 3]). scratch_pair:
  * device int array of max(nx, ny) entries. */

@@ -65,3 +65,38 @@ def test_cells_equal_brute_force(kind, k, n, nq):
         b, db = _search("cells", queries, p, k, self_)
         assert torch.equal(a, b)
         assert torch.equal(da.view(torch.int32), db.view(torch.int32))
+
+
+@pytest.mark.parametrize("kind", ["box", "plane", "point", "clusters", "lattice", "nan"])
+@pytest.mark.parametrize("sizes", [[(9001, 8000)], [(20_000, 9000), (1, 20_000), (17, 0), (0, 40), (5000, 4999)]])
+def test_chamfer_cells_equal_brute_force(kind, sizes):
+    """Neighbours bit for bit; the sums of n squared distances within n 2^-24."""
+    from empm_b200 import _native as N
+    L = N.lib()
+    rng = np.random.default_rng(3)
+    t = lambda a: torch.as_tensor(np.asarray(a, np.float32), device=DEV).contiguous()  # noqa: E731
+    xc, yc = [a for a, _ in sizes], [b for _, b in sizes]
+    x = t(np.concatenate([_cloud(rng, kind, a) for a in xc]))
+    y = t(np.concatenate([_cloud(rng, kind, b) for b in yc]))
+    off = lambda c: torch.as_tensor(np.cumsum([0] + c).astype(np.int32), device=DEV)  # noqa: E731
+    xo, yo = off(xc), off(yc)
+    res = []
+    for cells in (False, True):
+        s = torch.empty(2, len(sizes), device=DEV)
+        nx = torch.empty(len(x), dtype=torch.int32, device=DEV)
+        ny = torch.empty(len(y), dtype=torch.int32, device=DEV)
+        args = (x.data_ptr(), xo.data_ptr(), len(x), max(xc), y.data_ptr(), yo.data_ptr(), len(y), max(yc), len(sizes),
+                s[0].data_ptr(), s[1].data_ptr(), nx.data_ptr(), ny.data_ptr())
+        if cells:
+            nb = ctypes.c_size_t()
+            N.check(L.empm_chamfer_workspace(len(x), max(xc), len(y), max(yc), len(sizes), ctypes.byref(nb)))
+            assert nb.value > 0
+            work = torch.empty(nb.value, dtype=torch.uint8, device=DEV)
+            N.check(L.empm_chamfer_cells(*args, work.data_ptr(), nb.value, None))
+        else:
+            N.check(L.empm_chamfer(*args, None))
+        torch.cuda.synchronize()
+        res.append((s.double().cpu(), nx, ny))
+    assert torch.equal(res[0][1], res[1][1]) and torch.equal(res[0][2], res[1][2])
+    n = torch.as_tensor([xc, yc], dtype=torch.float64)
+    assert ((res[0][0] - res[1][0]).abs() <= 2 * n * 2.0 ** -24 * res[0][0] + 1e-30).all()
