@@ -126,7 +126,6 @@ struct EmpmCtx {
     float4*      grid_mom = nullptr;       // P2G accumulation (px, py, pz, m), blocked layout; zero between substeps
     float4*      grid_vel = nullptr;       // node velocity after the grid update, blocked layout
     unsigned char* flags = nullptr;        // touched node blocks of the current substep
-    int*         active = nullptr;         // [1 + blocks]: number of touched blocks, then their ids
     EmpmStep*    d_steps = nullptr;        // device copy of the step schedules
     unsigned*    d_status = nullptr;       // EMPM_STATUS_* bits
     cudaStream_t own_stream = nullptr;     // capture stream for the graph path
@@ -188,7 +187,6 @@ struct EmpmSegment {
     float*   vol = nullptr;       // [np]
     int*     sel = nullptr;       // [np]
     int*     pid = nullptr;       // [np] caller index of each position (cell order)
-    int*     max_count = nullptr; // device: largest touched-block count of the forward pass
     std::vector<EmpmStep> tables;
     EmpmStep* d_tables = nullptr; // device copy of tables, read by the segment's kernels
     bool     tables_on_device = false;

@@ -241,153 +241,60 @@ struct GridUpdateArgs {
     float4*        vel;      // node velocity after the boundary conditions (w = node mass)
     unsigned char* flags;    // touched blocks; cleared here
     Launch         L;
-    // optional store slot of the listed blocks (stored segments): per listed
-    // block its 64 node momenta, then its 64 node velocities; the list count
-    // and ids; a running maximum of the counts. A substep with more than
-    // store_cap listed blocks stores only its count.
+    // optional store slot of the touched blocks (stored segments): per block its
+    // 64 node momenta, then its 64 node velocities; the list count (zero before)
+    // and ids. Of more than store_cap blocks the others are only counted.
     float4*        store = nullptr;
     int*           store_list = nullptr;
     int            store_cap = 0;
-    int*           max_count = nullptr;
 };
 
-// One touched 4^3 block (64 nodes, two per lane of the calling warp):
-// normalisation, gravity, damping and boundary conditions.
-template <bool kKeep>
-__device__ __forceinline__ void grid_update_block(const GridUpdateArgs& a, int b, int lane) {
-    const int inst = find_instance_block(a.L, b);
-    const InstanceConsts* I = a.L.inst + inst;
-    const int G = __ldg(&I->G), NB = __ldg(&I->NB), boff = __ldg(&I->boff);
-    const float dx = __ldg(&I->dx), damping = __ldg(&I->damping);
-    const V3 g = v3(__ldg(&I->g[0]), __ldg(&I->g[1]), __ldg(&I->g[2]));
-    const EmpmStep& st = a.L.steps[(size_t)a.L.table * a.L.n_inst + inst];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int in_block = lane + 32 * h;
-        const long long node = ((long long)b << 6) | in_block;
-        const float4 m = a.mom[node];
-        if (!kKeep) a.mom[node] = make_float4(0.f, 0.f, 0.f, 0.f);
-        V3 v = grid_velocity(m, st.dt, g, damping);
-        if (st.n_colliders > 0) {
-            int i, j, k;
-            node_coords(((long long)(b - boff) << 6) | in_block, NB, i, j, k);
-            if (i < G && j < G && k < G) {
-                const long long dense = ((long long)i * G + j) * G + k;
-                apply_colliders(st, i, j, k, G, dx, dense, v);
-            }
-        }
-        a.vel[node] = make_float4(v.x, v.y, v.z, m.w);
-    }
-}
-
-// Grid update over the touched blocks. Each warp reads 32 block flags at a
-// time (coalesced), takes the set ones from a ballot and updates those
-// blocks; each lane clears its own flag afterwards, so no block-wide barrier
-// is needed. kKeep leaves the accumulation and the flags in place (the
-// adjoint replays the boundary conditions from the accumulated momentum).
-template <bool kKeep>
-__device__ __forceinline__ void grid_update_blocks(const GridUpdateArgs& a) {
-    const int nblocks = a.L.nblocks;
+// Calls f(block) for the touched blocks, a warp per call (all its lanes).
+// Touched blocks are neighbours, so a warp looks at blocks far apart: the marks of
+// its chunk c are those of blocks c, c + chunks, c + 2 chunks ..., as few per warp as
+// the launch's warps allow, and neighbouring warps read neighbouring bytes. That
+// spreads the work as a list of the touched blocks would, without the two launches
+// that reset and fill one (3.0 us of the 20 us of a 20k-particle substep; a list
+// written by the P2G kernels themselves took the population's 367 -> 445 us, for
+// the marks they then have to read). clear: the marks are reset.
+template <typename F>
+__device__ __forceinline__ void for_touched_blocks(unsigned char* marks, const Launch& L, bool clear, F f) {
     const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long base = warp * 32; base < nblocks; base += nwarps * 32) {
-        const long long b = base + lane;
-        const bool active = b < nblocks && a.flags[b] != 0;
-        unsigned mask = __ballot_sync(0xffffffffu, active);
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const int per = min(32, (L.nblocks + warps - 1) / warps);
+    const int chunks = (L.nblocks + per - 1) / per;
+    for (int c = warp; c < chunks; c += warps) {
+        const int b = c + lane * chunks;
+        const bool on = lane < per && b < L.nblocks && marks[b] != 0;
+        unsigned mask = __ballot_sync(0xffffffffu, on);
+        if (mask == 0u) continue;
+        if (on && clear) marks[b] = 0;
         while (mask) {
             const int j = __ffs(mask) - 1;
-            mask &= mask - 1;
-            grid_update_block<kKeep>(a, (int)(base + j), lane);
+            mask &= mask - 1u;
+            f(c + j * chunks);
         }
-        if (!kKeep && active) a.flags[b] = 0;
     }
 }
 
-__global__ void __launch_bounds__(256) k_grid_update_sparse(const GridUpdateArgs a) { grid_update_blocks<false>(a); }
-
-// Touched blocks -> list: active[0] counts them, active[1 + i] are their ids
-// (in no particular order) and active[1 + nblocks + i] their instances (the
-// lookup done once per block here rather than once per node by the update).
-// Clears the flags unless kKeep. active holds 1 + 2 * nblocks ints.
+// Grid update over the touched blocks, one warp per block and two nodes per lane:
+// normalisation, gravity, damping and boundary conditions. The accumulation is
+// cleared for the next substep; kKeep leaves it and the marks in place (the adjoint
+// replays the boundary conditions from the accumulated momentum).
 template <bool kKeep>
-__global__ void __launch_bounds__(256) k_collect_blocks(unsigned char* flags, int nblocks, int* active, const Launch L) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_grid_update(const GridUpdateArgs a) {
     const int lane = threadIdx.x & 31;
-    const bool on = b < nblocks && flags[b] != 0;
-    const unsigned m = __ballot_sync(0xffffffffu, on);
-    if (m == 0u) return;
-    const int leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(active, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (on) {
-        const int slot = base + __popc(m & ((1u << lane) - 1u));
-        active[1 + slot] = b;
-        active[1 + nblocks + slot] = find_instance_block(L, b);
-        if (!kKeep) flags[b] = 0;
-    }
-}
-
-// Grid update over the listed blocks, one thread per node (grid-stride).
-template <bool kKeep>
-__global__ void __launch_bounds__(256) k_grid_update_list(const GridUpdateArgs a, const int* active) {
-    const int count = __ldg(active);
-    const long long total = (long long)count * 64;
-    if (a.store && blockIdx.x == 0 && threadIdx.x == 0) {
-        a.store_list[0] = count;
-        if (a.max_count) atomicMax(a.max_count, count);
-    }
-    const bool save = a.store && count <= a.store_cap;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int b = __ldg(active + 1 + (idx >> 6));
-        const int in_block = (int)(idx & 63);
-        const int inst = __ldg(active + 1 + a.L.nblocks + (idx >> 6));
-        const InstanceConsts* I = a.L.inst + inst;
-        const EmpmStep& st = a.L.steps[(size_t)a.L.table * a.L.n_inst + inst];
-        const long long node = ((long long)b << 6) | in_block;
-        const float4 m = a.mom[node];
-        if (!kKeep) a.mom[node] = make_float4(0.f, 0.f, 0.f, 0.f);
-        V3 v = grid_velocity(m, st.dt, v3(__ldg(&I->g[0]), __ldg(&I->g[1]), __ldg(&I->g[2])), __ldg(&I->damping));
-        if (st.n_colliders > 0) {
-            const int G = __ldg(&I->G), NB = __ldg(&I->NB), boff = __ldg(&I->boff);
-            int i, j, k;
-            node_coords(((long long)(b - boff) << 6) | in_block, NB, i, j, k);
-            if (i < G && j < G && k < G) {
-                const long long dense = ((long long)i * G + j) * G + k;
-                apply_colliders(st, i, j, k, G, __ldg(&I->dx), dense, v);
-            }
+    for_touched_blocks(a.flags, a.L, !kKeep, [&](int b) {
+        const long long base = (long long)b << 6;
+        const float4 m0 = a.mom[base + lane];   // on their way while the instance is looked up
+        const float4 m1 = a.mom[base + lane + 32];
+        const int inst = find_instance_block(a.L, b);
+        int slot = 0;
+        if (a.store) {
+            if (lane == 0) slot = atomicAdd(a.store_list, 1);
+            slot = __shfl_sync(0xffffffffu, slot, 0);
         }
-        const float4 v4 = make_float4(v.x, v.y, v.z, m.w);
-        a.vel[node] = v4;
-        if (save) {
-            const long long slot = idx >> 6;
-            a.store[slot * 128 + in_block] = m;
-            a.store[slot * 128 + 64 + in_block] = v4;
-            if (in_block == 0) a.store_list[1 + slot] = b;
-        }
-    }
-}
-
-// Grid update over the listed blocks, one warp per block and two nodes per
-// lane (grid-stride over the list): the block id, its instance, the instance
-// constants and the step table are read once per warp, where
-// k_grid_update_list reads them once per node.
-template <bool kKeep>
-__global__ void __launch_bounds__(256) k_grid_update_warps(const GridUpdateArgs a, const int* active) {
-    const int count = __ldg(active);
-    if (a.store && blockIdx.x == 0 && threadIdx.x == 0) {
-        a.store_list[0] = count;
-        if (a.max_count) atomicMax(a.max_count, count);
-    }
-    const bool save = a.store && count <= a.store_cap;
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long slot = warp; slot < count; slot += nwarps) {
-        const int b = __ldg(active + 1 + slot);
-        const int inst = __ldg(active + 1 + a.L.nblocks + slot);
+        const bool save = a.store && slot < a.store_cap;
         const InstanceConsts* I = a.L.inst + inst;
         const EmpmStep& st = a.L.steps[(size_t)a.L.table * a.L.n_inst + inst];
         const V3 g = v3(__ldg(&I->g[0]), __ldg(&I->g[1]), __ldg(&I->g[2]));
@@ -396,9 +303,6 @@ __global__ void __launch_bounds__(256) k_grid_update_warps(const GridUpdateArgs 
         const int n_coll = st.n_colliders;
         const int G = __ldg(&I->G), NB = __ldg(&I->NB), boff = __ldg(&I->boff);
         const float dx = __ldg(&I->dx);
-        const long long base = (long long)b << 6;
-        const float4 m0 = a.mom[base + lane];
-        const float4 m1 = a.mom[base + lane + 32];
         if (!kKeep) {
             a.mom[base + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             a.mom[base + lane + 32] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -419,12 +323,12 @@ __global__ void __launch_bounds__(256) k_grid_update_warps(const GridUpdateArgs 
             const float4 v4 = make_float4(v.x, v.y, v.z, m.w);
             a.vel[base + in_block] = v4;
             if (save) {
-                a.store[slot * 128 + in_block] = m;
-                a.store[slot * 128 + 64 + in_block] = v4;
+                a.store[(long long)slot * 128 + in_block] = m;
+                a.store[(long long)slot * 128 + 64 + in_block] = v4;
             }
         }
         if (save && lane == 0) a.store_list[1 + slot] = b;
-    }
+    });
 }
 
 // -------------------------------------------------------------------------

@@ -43,22 +43,24 @@ __global__ void __launch_bounds__(128) k_restart_p2g(ParticleArrays P, const flo
 }
 
 // node displacement = accumulated (mass * displacement) / mass; zero the accumulator
-__global__ void __launch_bounds__(256) k_restart_grid(float4* mom, float4* vel, const int* active) {
-    const long long total = (long long)__ldg(active) * 64;
-    for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const long long node = ((long long)__ldg(active + 1 + (idx >> 6)) << 6) | (idx & 63);
-        const float4 m = mom[node];
-        mom[node] = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 v = make_float4(0.f, 0.f, 0.f, m.w);
-        if (m.w > 1e-15f) {
-            const float inv = 1.f / m.w;
-            v.x = m.x * inv;
-            v.y = m.y * inv;
-            v.z = m.z * inv;
+__global__ void __launch_bounds__(256) k_restart_grid(float4* mom, float4* vel, unsigned char* marks, const Launch L) {
+    const int lane = threadIdx.x & 31;
+    for_touched_blocks(marks, L, true, [&](int b) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const long long node = ((long long)b << 6) + lane + 32 * h;
+            const float4 m = mom[node];
+            mom[node] = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = make_float4(0.f, 0.f, 0.f, m.w);
+            if (m.w > 1e-15f) {
+                const float inv = 1.f / m.w;
+                v.x = m.x * inv;
+                v.y = m.y * inv;
+                v.z = m.z * inv;
+            }
+            vel[node] = v;
         }
-        vel[node] = v;
-    }
+    });
 }
 
 // PhysGaussian covariance update (update_cov, mpm_utils.py:306-326):

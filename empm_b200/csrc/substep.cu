@@ -250,7 +250,6 @@ extern "C" int empm_batch_create(const EmpmModelParams* params, const int* n_par
     if (e == cudaSuccess) e = cudaMalloc(&ctx->grid_mom, grid_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->grid_vel, grid_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->flags, (size_t)blocks);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->active, sizeof(int) * (2 * (size_t)blocks + 1));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->grid_mom, 0, grid_bytes);
     if (e == cudaSuccess) e = cudaMemset(ctx->grid_vel, 0, grid_bytes);
@@ -284,7 +283,7 @@ extern "C" int empm_ctx_destroy(EmpmCtx* ctx) {
     for (cudaEvent_t ev : ctx->timing_events) cudaEventDestroy(ev);
     free_sorted(ctx->sb);
     free_adjoint(ctx->adj);
-    void* ptrs[] = {ctx->d_inst, ctx->grid_mom, ctx->grid_vel, ctx->flags, ctx->active, ctx->d_steps, ctx->d_status};
+    void* ptrs[] = {ctx->d_inst, ctx->grid_mom, ctx->grid_vel, ctx->flags, ctx->d_steps, ctx->d_status};
     for (void* q : ptrs) if (q) cudaFree(q);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->ev_a) cudaEventDestroy(ctx->ev_a);
@@ -356,14 +355,11 @@ extern "C" int empm_batch_reserve(EmpmCtx* ctx, int max_particles, long long max
         cudaFree(ctx->grid_mom);
         cudaFree(ctx->grid_vel);
         cudaFree(ctx->flags);
-        cudaFree(ctx->active);
         ctx->grid_mom = ctx->grid_vel = nullptr;
         ctx->flags = nullptr;
-        ctx->active = nullptr;
         CK(cudaMalloc(&ctx->grid_mom, grid_bytes), "reserve grid");
         CK(cudaMalloc(&ctx->grid_vel, grid_bytes), "reserve grid");
         CK(cudaMalloc(&ctx->flags, (size_t)max_blocks), "reserve grid");
-        CK(cudaMalloc(&ctx->active, sizeof(int) * (2 * (size_t)max_blocks + 1)), "reserve grid");
         CK(cudaMemset(ctx->grid_mom, 0, grid_bytes), "reserve grid");
         CK(cudaMemset(ctx->grid_vel, 0, grid_bytes), "reserve grid");
         CK(cudaMemset(ctx->flags, 0, (size_t)max_blocks), "reserve grid");
@@ -557,20 +553,11 @@ static ParticleArrays particle_arrays(float* base, int n) {
     return a;
 }
 
-// Grid update of one substep: the touched blocks are collected into a list
-// (the count is reset first), then every node of the listed blocks is
-// updated by its own thread. kKeep leaves the momentum and the flags in place.
 // Threads per block of the P2G kernels: the kernel's usual size, or 64 when
 // that would leave fewer than two blocks per SM (small instances would
 // otherwise run on a fraction of the SMs; measured 16.7 -> 15.0 us for 20k
 // particles; G2P measured no better). The kernels use no block-wide
 // synchronisation, so any multiple of the warp size works.
-// 1: the grid update runs one warp per touched block (k_grid_update_warps),
-// 0: one thread per node (k_grid_update_list)
-#ifndef EMPM_GRID_UPDATE_WARPS
-#define EMPM_GRID_UPDATE_WARPS 1
-#endif
-
 static int particle_threads(const EmpmCtx* ctx, long long n, int usual) {
     return blocks_for(n, usual) >= 2LL * ctx->sm_count ? usual : 64;
 }
@@ -586,17 +573,17 @@ static int uniform_material(const EmpmCtx* ctx) {
     return m;
 }
 
-// Optional store slot for launch_grid_update_list (stored segments).
+// Optional store slot for launch_grid_update_on (stored segments).
 struct GridStoreSlot {
     float4* blocks;
     int*    list;
     int     cap;
-    int*    max_count;
 };
 
+// Grid update of one substep. kKeep leaves the momentum and the marks in place.
 template <bool kKeep>
-static int launch_grid_update_list(EmpmCtx* ctx, const Launch& L, cudaStream_t stream,
-                                   const GridStoreSlot* store = nullptr) {
+static int launch_grid_update_on(EmpmCtx* ctx, const Launch& L, cudaStream_t stream,
+                                 const GridStoreSlot* store = nullptr) {
     GridUpdateArgs g;
     g.mom = ctx->grid_mom;
     g.vel = ctx->grid_vel;
@@ -606,24 +593,17 @@ static int launch_grid_update_list(EmpmCtx* ctx, const Launch& L, cudaStream_t s
         g.store = store->blocks;
         g.store_list = store->list;
         g.store_cap = store->cap;
-        g.max_count = store->max_count;
     }
-    CK(cudaMemsetAsync(ctx->active, 0, sizeof(int), stream), "reset touched-block count");
-    k_collect_blocks<kKeep><<<blocks_for(ctx->nblocks, 256), 256, 0, stream>>>(ctx->flags, (int)ctx->nblocks,
-                                                                               ctx->active, L);
-    CK(cudaGetLastError(), "k_collect_blocks");
-#if EMPM_GRID_UPDATE_WARPS
-    k_grid_update_warps<kKeep><<<ctx->sm_count * 8, 256, 0, stream>>>(g, ctx->active);
-#else
-    k_grid_update_list<kKeep><<<ctx->sm_count * 8, 256, 0, stream>>>(g, ctx->active);
-#endif
-    CK(cudaGetLastError(), "k_grid_update_list");
+    // 8 warps per CTA, a warp per block at most
+    const int ctas = std::max(1, std::min(ctx->sm_count * 8, blocks_for(ctx->nblocks, 8)));
+    k_grid_update<kKeep><<<ctas, 256, 0, stream>>>(g);
+    CK(cudaGetLastError(), "k_grid_update");
     return EMPM_OK;
 }
 
 static int launch_grid_update(EmpmCtx* ctx, int table, cudaStream_t stream) {
     timing_mark(ctx, 1, 0, stream);
-    const int rc = launch_grid_update_list<false>(ctx, make_launch(ctx, table), stream);
+    const int rc = launch_grid_update_on<false>(ctx, make_launch(ctx, table), stream);
     timing_mark(ctx, 1, 1, stream);
     return rc;
 }
@@ -1410,7 +1390,6 @@ struct SegmentData {
     int* glist = nullptr;      // n_steps x (1 + cap_blocks)
     float* fe = nullptr;       // n_steps x f9 planes
     size_t cap_blocks = 0;     // grid blocks per substep slot
-    int* max_count = nullptr;  // running maximum of the touched-block counts, or NULL
     const EmpmStep* steps = nullptr;   // device step tables: [n_steps) as run, [n_steps, 2 n_steps) for recomputing
     MaterialArrays base;
 };
@@ -1439,6 +1418,8 @@ static int segment_forward(EmpmCtx* ctx, const SegmentData& d, cudaStream_t s) {
     // previous substep and the stress + P2G of this one run as one kernel
     // that writes the stored state, snapshot and elastic F itself
     const bool fused = d.store && d.sorted && ctx->fuse && d.n_steps > 1;
+    if (d.store)   // each substep's grid update counts its blocks from zero
+        CK(cudaMemset2DAsync(d.glist, (d.cap_blocks + 1) * sizeof(int), 0, sizeof(int), d.n_steps, s), "block counts");
     for (int k = 0; k < d.n_steps; ++k) {
         const ParticleArrays Pin = particle_arrays(d.states + (size_t)k * state_floats, n);
         const ParticleArrays Pout = particle_arrays(d.states + (size_t)(k + 1) * state_floats, n);
@@ -1481,8 +1462,7 @@ static int segment_forward(EmpmCtx* ctx, const SegmentData& d, cudaStream_t s) {
         slot.blocks = d.gsave + (size_t)k * d.cap_blocks * 128;
         slot.list = d.glist + (size_t)k * (d.cap_blocks + 1);
         slot.cap = (int)d.cap_blocks;
-        slot.max_count = d.max_count;
-        const int rc = launch_grid_update_list<false>(ctx, Lk, s, &slot);
+        const int rc = launch_grid_update_on<false>(ctx, Lk, s, &slot);
         if (rc) return rc;
         timing_mark(ctx, 1, 1, s);
         if (fused && k + 1 < d.n_steps) continue;   // the next fused kernel runs this G2P
@@ -1540,7 +1520,7 @@ static int segment_reverse(EmpmCtx* ctx, const SegmentData& d, ParticleArrays Gp
             timing_mark(ctx, 0, 1, s);
             CK(cudaGetLastError(), "P2G (adjoint recompute)");
             timing_mark(ctx, 1, 0, s);
-            const int rc = launch_grid_update_list<true>(ctx, Lrec, s);
+            const int rc = launch_grid_update_on<true>(ctx, Lrec, s);
             timing_mark(ctx, 1, 1, s);
             if (rc) return rc;
         }
@@ -1830,12 +1810,12 @@ static size_t segment_bytes(size_t np, size_t cap_blocks, int n_steps) {
 }
 
 static size_t segment_bytes(const EmpmCtx* ctx, size_t np, size_t cap_blocks, int n_steps) {
-    return segment_bytes(np, cap_blocks, n_steps) + (size_t)n_steps * ctx->n_inst * sizeof(EmpmStep) + sizeof(int);
+    return segment_bytes(np, cap_blocks, n_steps) + (size_t)n_steps * ctx->n_inst * sizeof(EmpmStep);
 }
 
 static void segment_free(EmpmSegment* seg) {
     void* ptrs[] = {seg->states, seg->mats, seg->gsave, seg->glist, seg->fe, seg->vol, seg->sel, seg->pid,
-                    seg->max_count, seg->d_tables};
+                    seg->d_tables};
     for (void* q : ptrs) if (q) cudaFree(q);
     if (seg->fwd_exec) cudaGraphExecDestroy(seg->fwd_exec);
     if (seg->rev_exec) cudaGraphExecDestroy(seg->rev_exec);
@@ -1844,7 +1824,7 @@ static void segment_free(EmpmSegment* seg) {
     seg->tables_on_device = false;
     seg->states = seg->mats = seg->fe = seg->vol = nullptr;
     seg->gsave = nullptr;
-    seg->glist = seg->sel = seg->pid = seg->max_count = nullptr;
+    seg->glist = seg->sel = seg->pid = nullptr;
 }
 
 // block slots per substep: 0 (or more than the context has) means all of them
@@ -1882,7 +1862,6 @@ extern "C" int empm_segment_create(EmpmCtx* ctx, int n_steps, int block_cap, Emp
     if (e == cudaSuccess) e = cudaMalloc(&seg->vol, np * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&seg->sel, np * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&seg->pid, np * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&seg->max_count, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&seg->d_tables, k * (size_t)ctx->n_inst * sizeof(EmpmStep));
     if (e != cudaSuccess) {
         segment_free(seg);
@@ -1929,7 +1908,6 @@ static SegmentData segment_data(const EmpmSegment* seg) {
     d.glist = seg->glist;
     d.fe = seg->fe;
     d.cap_blocks = seg->block_cap;
-    d.max_count = seg->max_count;
     d.steps = seg->d_tables;
     d.base.vol = seg->vol;
     d.base.mu = d.base.lam = d.base.ys = nullptr;
@@ -1980,7 +1958,6 @@ extern "C" int empm_segment_forward(EmpmCtx* ctx, EmpmSegment* seg, const EmpmPa
     AdjointBuffers& ab = ctx->adj;
     const size_t np = seg->np;
     const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
-    CK(cudaMemsetAsync(seg->max_count, 0, sizeof(int), s), "reset touched-block maximum");
     ctx->resident = false;   // a sort here reuses the rollout's sorted buffers
     seg->sorted = ctx->sort_every > 0;
     seg->has_sel = seg->sorted || mat->selection != nullptr;
@@ -2059,9 +2036,12 @@ extern "C" int empm_segment_blocks(EmpmSegment* seg, int* max_touched, int* bloc
     if (!seg->checked) {
         int m = 0;
         if (seg->n > 0) {
-            CK(cudaMemcpyAsync(&m, seg->max_count, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream),
-               "read touched-block maximum");
-            CK(cudaStreamSynchronize((cudaStream_t)stream), "read touched-block maximum");
+            std::vector<int> counts(seg->n_steps);
+            CK(cudaMemcpy2DAsync(counts.data(), sizeof(int), seg->glist, (seg->block_cap + 1) * sizeof(int), sizeof(int),
+                                 seg->n_steps, cudaMemcpyDeviceToHost, (cudaStream_t)stream),
+               "read touched-block counts");
+            CK(cudaStreamSynchronize((cudaStream_t)stream), "read touched-block counts");
+            m = *std::max_element(counts.begin(), counts.end());
         }
         seg->max_touched = m;
         seg->checked = true;
@@ -2142,11 +2122,7 @@ extern "C" int empm_restart_F(EmpmCtx* ctx, EmpmParticles* p, const float* targe
     const ParticleArrays P = particle_arrays(p, n);
     k_restart_p2g<<<blocks_for(n, 128), 128, 0, s>>>(P, target, selection, L, ctx->grid_mom, ctx->flags);
     CK(cudaGetLastError(), "k_restart_p2g");
-    CK(cudaMemsetAsync(ctx->active, 0, sizeof(int), s), "reset touched-block count");
-    k_collect_blocks<false><<<blocks_for(ctx->nblocks, 256), 256, 0, s>>>(ctx->flags, (int)ctx->nblocks, ctx->active,
-                                                                          L);
-    CK(cudaGetLastError(), "k_collect_blocks");
-    k_restart_grid<<<ctx->sm_count * 8, 256, 0, s>>>(ctx->grid_mom, ctx->grid_vel, ctx->active);
+    k_restart_grid<<<ctx->sm_count * 8, 256, 0, s>>>(ctx->grid_mom, ctx->grid_vel, ctx->flags, L);
     CK(cudaGetLastError(), "k_restart_grid");
     k_restart_g2p<<<blocks_for(n, 128), 128, 0, s>>>(P, target, selection, L, ctx->grid_vel, cov);
     CK(cudaGetLastError(), "k_restart_g2p");
@@ -2329,10 +2305,8 @@ extern "C" int empm_substep_noalloc(const EmpmModelParams* params, const EmpmPar
     g.vel = vel;
     g.flags = P->flags;
     g.L = L;
-    long long nb = (nblocks + 3) / 4;
-    if (nb > 148 * 8) nb = 148 * 8;
-    k_grid_update_sparse<<<(int)nb, 256, 0, s>>>(g);
-    CK(cudaGetLastError(), "k_grid_update_sparse (allocation-free)");
+    k_grid_update<false><<<std::min(148 * 8, blocks_for(nblocks, 8)), 256, 0, s>>>(g);
+    CK(cudaGetLastError(), "k_grid_update (allocation-free)");
     if (n_particles > 0) {
         k_g2p_direct<<<blocks_for(n_particles, 128), 128, 0, s>>>(Pin, Fe, M, Pout, L, vel);
         CK(cudaGetLastError(), "k_g2p_direct (allocation-free)");
