@@ -12,7 +12,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "libempm_b200.so")
 
 EMPM_OK = 0
-ROLLOUT_GRAPH, ROLLOUT_RESUME, ROLLOUT_KEEP = 1, 2, 4
+ROLLOUT_GRAPH, ROLLOUT_RESUME, ROLLOUT_KEEP, ROLLOUT_TAPE = 1, 2, 4, 8
 EMPM_ERR_INVALID, EMPM_ERR_CUDA, EMPM_ERR_OOM, EMPM_ERR_UNSUPPORTED = -1, -2, -3, -4
 EMPM_MAX_COLLIDERS = 16
 EMPM_MAX_MODIFIERS = 8

@@ -307,7 +307,7 @@ class CheckpointedRollout:
                 self.ckpts.append(_Checkpoint(s0, cur._x4.clone(), cur._v4.clone(), cur._C.clone(),
                                               cur._F_trial.clone(), model.mu.clone(), model.lam.clone(),
                                               model.yield_stress.clone()))
-                res = solver.rollout(model, cur, other, self.dt, L, schedule=(seg, times[s1]))
+                res = solver._rollout(model, cur, other, self.dt, L, schedule=(seg, times[s1]), flags=N.ROLLOUT_TAPE)
                 if res is not cur:
                     cur, other = other, cur
             if (s1 - 1) in record_set:

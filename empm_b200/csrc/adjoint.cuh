@@ -533,13 +533,11 @@ __global__ void __launch_bounds__(128, EMPM_ADJ_P2G_MIN_CTAS) k_adj_p2g(const Ad
     a.g_mass[p] += gmass;
     const M3 g_tau = (-vol * dt) * gSv;
 
-    M3 tau;
-    const SpectralGrad sg = constitutive_adjoint<MAT>(f9_load(a.P.F, p), __ldg(a.M.mu + p), __ldg(a.M.lam + p),
-                                                      __ldg(a.M.ys + p), dt, *c.ms, f9_load(a.gFe, p), g_tau,
-                                                      a.g_mu[p], a.g_lam[p], a.g_ys[p], tau);
+    SpectralEval e;
+    spectral_eval<MAT>(f9_load(a.P.F, p), __ldg(a.M.mu + p), __ldg(a.M.lam + p), __ldg(a.M.ys + p), dt, *c.ms, e);
     {
         // sum_n H_n Sv^T gmv_n, component a = sum_b dot(column b of Sv, sum_n H_n[a][b] gmv_n)
-        const M3 Sv = (-vol) * tau;
+        const M3 Sv = (-vol) * spectral_tau(e);
         const V3 c0 = v3(Sv.m[0], Sv.m[3], Sv.m[6]);
         const V3 c1 = v3(Sv.m[1], Sv.m[4], Sv.m[7]);
         const V3 c2 = v3(Sv.m[2], Sv.m[5], Sv.m[8]);
@@ -550,6 +548,8 @@ __global__ void __launch_bounds__(128, EMPM_ADJ_P2G_MIN_CTAS) k_adj_p2g(const Ad
         const float4 gxg = __ldg(a.gx + p);
         a.G.x[p] = make_float4(gxa.x + gxg.x, gxa.y + gxg.y, gxa.z + gxg.z, 0.f);
     }
+
+    const SpectralGrad sg = spectral_adjoint(e, f9_load(a.gFe, p), g_tau, a.g_mu[p], a.g_lam[p], a.g_ys[p]);
     f9_store(a.G.F, p, sg.gFt);
     a.g_mu[p] = sg.g_mu;
     a.g_lam[p] = sg.g_lam;

@@ -186,7 +186,7 @@ __device__ __forceinline__ bool prepare_particle(const ParticleArrays& P, const 
         if (apply_modifiers(st, mi, x, xm.w, v)) P.v[p] = make_float4(v.x, v.y, v.z, vv.w);
     }
     float mu = __ldg(M.mu + p), lam = __ldg(M.lam + p), ys = __ldg(M.ys + p);
-    const ConstitutiveOut co = constitutive<MAT>(f9_load(P.F, p), mu, lam, ys, st.dt, *c.ms);
+    const ConstitutiveOut co = constitutive_general<MAT>(f9_load(P.F, p), mu, lam, ys, st.dt, *c.ms);
     f9_store(Fe, p, co.F);
     if (co.mat_changed) { M.mu[p] = mu; M.lam[p] = lam; M.ys[p] = ys; }
     q.st = make_stencil(x, c.inv_dx);
@@ -702,7 +702,8 @@ __global__ void k_unsort(const UnsortArgs a) {
 // modifiers are written, and the contributions
 //   (weight * mass) (v + C dpos) - dt vol stress dweight, dpos = ((i, j, k) - fx) dx,
 // go into the grid: a = v - dx C fx, B = dx C and S = -dt inv_dx vol stress.
-template <int MAT, int NT>
+// TAPE: for a tape, with the general constitutive update.
+template <int MAT, bool TAPE, int NT>
 __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid, const StepConsts& c,
                                           const EmpmStep& sp, const MaterialArrays& M, int p, V3 x, float mass, V3 v,
                                           const M3& C, const M3& Ft, float mu, float lam, float ys, float vol,
@@ -724,7 +725,8 @@ __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid,
         for (int a = 0; a < 3; ++a) fx[a] = base_frac(xs[a], c.inv_dx, b[a]);
         const M3 B = (mass * c.dx) * damp_affine(C, c.rpic);
         cell_scatter_put(sh, cell.slot, fx, mass, mass * v - B * v3(fx[0], fx[1], fx[2]), B);
-        const ConstitutiveOut co = constitutive<MAT>(Ft, mu, lam, ys, sp.dt, *c.ms);
+        const ConstitutiveOut co = TAPE ? constitutive_general<MAT>(Ft, mu, lam, ys, sp.dt, *c.ms)
+                                        : constitutive<MAT>(Ft, mu, lam, ys, sp.dt, *c.ms);
         f9_store(Fe, p, co.F);
         if (co.mat_changed) { M.mu[p] = mu; M.lam[p] = lam; M.ys[p] = ys; }
         cell_scatter_put(sh, cell.slot, (sp.dt * c.inv_dx * -vol) * co.tau);
@@ -736,7 +738,7 @@ __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid,
     cell_scatter(sh, cell, grid, flags);
 }
 
-template <int NT, int MAT, int MINB>
+template <int NT, int MAT, int MINB, bool TAPE>
 __global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
                                                         float4* grid, unsigned char* flags) {
     __shared__ CellScatter<true, NT> sh;
@@ -759,7 +761,7 @@ __global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, Materi
         ys = __ldg(M.ys + p);
         vol = __ldg(M.vol + p);
     }
-    p2g_cells<MAT>(sh, valid, c, sp, M, p, v3(xm.x, xm.y, xm.z), xm.w, v3(vv.x, vv.y, vv.z), C, F, mu, lam, ys, vol,
+    p2g_cells<MAT, TAPE>(sh, valid, c, sp, M, p, v3(xm.x, xm.y, xm.z), xm.w, v3(vv.x, vv.y, vv.z), C, F, mu, lam, ys, vol,
                    Fe, sp.n_modifiers > 0 ? P.v : nullptr, grid, flags);
 }
 
@@ -778,7 +780,7 @@ __global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, Materi
 // full state. Held instances (step-table hold) must stay held once held within
 // the run: when a particle's instance becomes held at substep s, its state
 // after the G2P of s-1 is written in full, then left alone.
-template <int NT, int MAT, int MINB>
+template <int NT, int MAT, int MINB, bool TAPE>
 __global__ void __launch_bounds__(NT, MINB) k_g2p2g(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
                                                     int g2p_table, const float4* vel, float4* mom,
                                                     unsigned char* flags) {
@@ -807,7 +809,7 @@ __global__ void __launch_bounds__(NT, MINB) k_g2p2g(ParticleArrays P, MaterialAr
             f9_store(P.F, p, Fn);
         }
     }
-    p2g_cells<MAT>(sh, valid, c, sp, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, Fe, nullptr, mom,
+    p2g_cells<MAT, TAPE>(sh, valid, c, sp, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, Fe, nullptr, mom,
                    flags);
 }
 
@@ -828,7 +830,7 @@ struct SegmentStoreArgs {
     long long      np;
 };
 
-template <int NT, int MAT, int MINB>
+template <int NT, int MAT, int MINB, bool TAPE>
 __global__ void __launch_bounds__(NT, MINB) k_g2p2g_store(MaterialArrays M, Launch L, int g2p_table,
                                                           const float4* vel, float4* mom, unsigned char* flags,
                                                           SegmentStoreArgs a) {
@@ -862,7 +864,7 @@ __global__ void __launch_bounds__(NT, MINB) k_g2p2g_store(MaterialArrays M, Laun
         f9_store(a.cur.C, p, m3_zero());
         f9_store(a.cur.F, p, m3_identity());
     }
-    p2g_cells<MAT>(sh, valid, c, *c.step, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, a.fe_cur,
+    p2g_cells<MAT, true>(sh, valid, c, *c.step, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, a.fe_cur,
                    a.cur.v, mom, flags);
 }
 
@@ -871,40 +873,42 @@ __global__ void __launch_bounds__(NT, MINB) k_g2p2g_store(MaterialArrays M, Laun
 constexpr int kCellThreads = EMPM_CELL_THREADS;
 constexpr int kCellThreadsFew = 64;
 
-// One launch of a kernel template <NT, MAT, MINB>; material: the id every
+// One launch of a kernel template <NT, MAT, MINB, TAPE>; material: the id every
 // instance of the launch uses (plasticine 5 and jelly 0 have kernels without
 // the other materials' code), or -1 when they differ.
-#define EMPM_CELL_LAUNCH(kernel, min_ctas, n, few, material, stream, ...)                                              \
+#define EMPM_CELL_LAUNCH(kernel, min_ctas, tape, n, few, material, stream, ...)                                        \
     do {                                                                                                             \
         const int nt_ = (few) ? kCellThreadsFew : kCellThreads;                                                      \
         const int g_ = ((n) + nt_ - 1) / nt_;                                                                        \
         if (few) {                                                                                                   \
-            if ((material) == 5) kernel<kCellThreadsFew, 5, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                 \
-            else if ((material) == 0) kernel<kCellThreadsFew, 0, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);            \
-            else kernel<kCellThreadsFew, -1, 1><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                                \
+            if ((material) == 5) kernel<kCellThreadsFew, 5, 1, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                 \
+            else if ((material) == 0) kernel<kCellThreadsFew, 0, 1, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);            \
+            else kernel<kCellThreadsFew, -1, 1, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                                \
         } else {                                                                                                     \
-            if ((material) == 5) kernel<kCellThreads, 5, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);             \
-            else if ((material) == 0) kernel<kCellThreads, 0, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);        \
-            else kernel<kCellThreads, -1, min_ctas><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                            \
+            if ((material) == 5) kernel<kCellThreads, 5, min_ctas, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);             \
+            else if ((material) == 0) kernel<kCellThreads, 0, min_ctas, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);        \
+            else kernel<kCellThreads, -1, min_ctas, tape><<<g_, nt_, 0, stream>>>(__VA_ARGS__);                            \
         }                                                                                                            \
     } while (0)
 
 static inline void launch_g2p2g_store(bool few, cudaStream_t s, const MaterialArrays& M, const Launch& L,
                                       int g2p_table, const float4* vel, float4* mom, unsigned char* flags,
                                       const SegmentStoreArgs& a, int material) {
-    EMPM_CELL_LAUNCH(k_g2p2g_store, EMPM_FUSED_MIN_CTAS, L.n_total, few, material, s, M, L, g2p_table, vel, mom, flags, a);
+    EMPM_CELL_LAUNCH(k_g2p2g_store, EMPM_FUSED_MIN_CTAS, true, L.n_total, few, material, s, M, L, g2p_table, vel, mom, flags, a);
 }
 
+template <bool TAPE>
 static inline void launch_g2p2g(bool few, cudaStream_t s, const ParticleArrays& P, const MaterialArrays& M,
                                 const F9Planes& Fe, const Launch& L, int g2p_table, const float4* vel, float4* mom,
                                 unsigned char* flags, int material) {
-    EMPM_CELL_LAUNCH(k_g2p2g, EMPM_FUSED_MIN_CTAS, L.n_total, few, material, s, P, M, Fe, L, g2p_table, vel, mom, flags);
+    EMPM_CELL_LAUNCH(k_g2p2g, EMPM_FUSED_MIN_CTAS, TAPE, L.n_total, few, material, s, P, M, Fe, L, g2p_table, vel, mom, flags);
 }
 
+template <bool TAPE>
 static inline void launch_p2g_cells(bool few, cudaStream_t s, const ParticleArrays& P, const MaterialArrays& M,
                                     const F9Planes& Fe, const Launch& L, float4* mom, unsigned char* flags,
                                     int material) {
-    EMPM_CELL_LAUNCH(k_p2g_cells, EMPM_P2G_MIN_CTAS, L.n_total, few, material, s, P, M, Fe, L, mom, flags);
+    EMPM_CELL_LAUNCH(k_p2g_cells, EMPM_P2G_MIN_CTAS, TAPE, L.n_total, few, material, s, P, M, Fe, L, mom, flags);
 }
 
 // -------------------------------------------------------------------------

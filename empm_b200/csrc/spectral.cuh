@@ -320,127 +320,4 @@ EMPM_HD SpectralGrad spectral_adjoint(const SpectralEval& e, const M3& g_Fe, con
     return g;
 }
 
-// The adjoint of fcr_elastic's branch (F_e = F, tau = 2 mu (F - R) F^T +
-// lam J (J - 1) I, scalars passed through) without a decomposition. With F = R S
-// and dR = R [w]x the rotation follows (tr S I - S) w = axial(R^T dF - dF^T R), so
-// for G = sym(g_tau) and y solving (tr S I - S) y = axial(A - A^T), A = R^T G F,
-//   gF = gF_e + 2 mu (G F + G (F - R) - R [y]x) + lam tr G (2 J - 1) cof F.
-// The strain enters as F - R, not as singular values with the rounding of a
-// decomposition, whose bias of 1e-7 is 1e-3 of a strain of 1e-4.
-EMPM_HD SpectralGrad fcr_elastic_adjoint(const M3& F, const M3& R, float J1, float mu, float lam, const M3& g_Fe,
-                                         const M3& g_tau, float g_mu_out, float g_lam_out, float g_ys_out) {
-    const M3 G = 0.5f * (g_tau + transpose(g_tau));
-    const M3 D = F - R;
-    const M3 H = G * F;
-    const M3 A = transpose(R) * H;
-    const V3 a = v3(A.m[7] - A.m[5], A.m[2] - A.m[6], A.m[3] - A.m[1]);
-    // tr S I - S, S = R^T F symmetric
-    const V3 r0 = col(R, 0), r1 = col(R, 1), r2 = col(R, 2), f0 = col(F, 0), f1 = col(F, 1), f2 = col(F, 2);
-    const float s00 = dot(r0, f0), s11 = dot(r1, f1), s22 = dot(r2, f2);
-    const float m00 = s11 + s22, m11 = s00 + s22, m22 = s00 + s11;
-    const float m01 = -0.5f * (dot(r0, f1) + dot(r1, f0)), m02 = -0.5f * (dot(r0, f2) + dot(r2, f0)),
-                m12 = -0.5f * (dot(r1, f2) + dot(r2, f1));
-    const float c00 = m11 * m22 - m12 * m12, c01 = m02 * m12 - m01 * m22, c02 = m01 * m12 - m02 * m11;
-    const float c11 = m00 * m22 - m02 * m02, c12 = m01 * m02 - m00 * m12, c22 = m00 * m11 - m01 * m01;
-    const float inv = 1.f / (m00 * c00 + m01 * c01 + m02 * c02);
-    const V3 y = inv * v3(c00 * a.x + c01 * a.y + c02 * a.z, c01 * a.x + c11 * a.y + c12 * a.z,
-                          c02 * a.x + c12 * a.y + c22 * a.z);
-    const float trG = G.m[0] + G.m[4] + G.m[8];
-    const float p = lam * trG * (1.f + 2.f * J1), m2 = 2.f * mu;
-    const M3 GD = G * D;
-    SpectralGrad g;
-    // R [y]x: row i is R_i x y taken column by column
-    const M3 cofF = [&] {
-        M3 c;
-        c.m[0] = F.m[4] * F.m[8] - F.m[5] * F.m[7];
-        c.m[1] = F.m[5] * F.m[6] - F.m[3] * F.m[8];
-        c.m[2] = F.m[3] * F.m[7] - F.m[4] * F.m[6];
-        c.m[3] = F.m[2] * F.m[7] - F.m[1] * F.m[8];
-        c.m[4] = F.m[0] * F.m[8] - F.m[2] * F.m[6];
-        c.m[5] = F.m[1] * F.m[6] - F.m[0] * F.m[7];
-        c.m[6] = F.m[1] * F.m[5] - F.m[2] * F.m[4];
-        c.m[7] = F.m[2] * F.m[3] - F.m[0] * F.m[5];
-        c.m[8] = F.m[0] * F.m[4] - F.m[1] * F.m[3];
-        return c;
-    }();
-    float hd = 0.f;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float x0 = R.m[3 * i], x1 = R.m[3 * i + 1], x2 = R.m[3 * i + 2];
-        const float q[3] = {x1 * y.z - x2 * y.y, x2 * y.x - x0 * y.z, x0 * y.y - x1 * y.x};
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int e = 3 * i + j;
-            g.gFt.m[e] = g_Fe.m[e] + m2 * ((H.m[e] + GD.m[e]) - q[j]) + p * cofF.m[e];
-            hd += H.m[e] * D.m[e];
-        }
-    }
-    g.g_mu = g_mu_out + 2.f * hd;
-    g.g_lam = g_lam_out + trG * (1.f + J1) * J1;
-    g.g_ys = g_ys_out;
-    return g;
-}
-
-// Constitutive adjoint of one particle: tau is the (forward) stress. In the
-// kernels compiled for jelly (0) and plasticine (5) elastic particles take the
-// branch above, and the others go through the decomposition and the dual-number
-// map in a call of its own, so that the kernel's registers are those of the common
-// path (200k-particle substep: 43.4 -> 36.4 us).
-struct SpectralCall {
-    M3 F, g_Fe, g_tau;          // in
-    float mu, lam, ys;
-    float g_mu, g_lam, g_ys;    // in: of the updated scalars; out: of those before
-    M3 tau, gFt;                // out
-};
-template <int MAT>
-#ifdef __CUDACC__
-__host__ __device__ __noinline__
-#else
-inline
-#endif
-void spectral_call(SpectralCall* io, float dt, const MaterialScalars* ms) {
-    SpectralEval e;
-    spectral_eval<MAT>(io->F, io->mu, io->lam, io->ys, dt, *ms, e);
-    io->tau = spectral_tau(e);
-    const SpectralGrad g = spectral_adjoint(e, io->g_Fe, io->g_tau, io->g_mu, io->g_lam, io->g_ys);
-    io->gFt = g.gFt;
-    io->g_mu = g.g_mu;
-    io->g_lam = g.g_lam;
-    io->g_ys = g.g_ys;
-}
-
-template <int MAT>
-EMPM_HD SpectralGrad constitutive_adjoint(const M3& F, float mu, float lam, float ys, float dt,
-                                          const MaterialScalars& ms, const M3& g_Fe, const M3& g_tau, float g_mu,
-                                          float g_lam, float g_ys, M3& tau) {
-    if (MAT != 0 && MAT != 5) {   // nearly all particles take the decomposition: not a call
-        SpectralEval e;
-        spectral_eval<MAT>(F, mu, lam, ys, dt, ms, e);
-        tau = spectral_tau(e);
-        return spectral_adjoint(e, g_Fe, g_tau, g_mu, g_lam, g_ys);
-    }
-    M3 R;
-    float J1;
-    if (fcr_elastic(F, mu, lam, ys, MAT == 5, tau, R, J1))
-        return fcr_elastic_adjoint(F, R, J1, mu, lam, g_Fe, g_tau, g_mu, g_lam, g_ys);
-    SpectralCall io;
-    io.F = F;
-    io.g_Fe = g_Fe;
-    io.g_tau = g_tau;
-    io.mu = mu;
-    io.lam = lam;
-    io.ys = ys;
-    io.g_mu = g_mu;
-    io.g_lam = g_lam;
-    io.g_ys = g_ys;
-    spectral_call<MAT>(&io, dt, &ms);
-    tau = io.tau;
-    SpectralGrad g;
-    g.gFt = io.gFt;
-    g.g_mu = io.g_mu;
-    g.g_lam = io.g_lam;
-    g.g_ys = io.g_ys;
-    return g;
-}
-
 }  // namespace empm

@@ -693,6 +693,7 @@ static int ensure_sorted_buffers(EmpmCtx* ctx) {
 struct SortedState {
     int pc = 0;   // particle buffer holding the current state
     int mc = 0;   // material buffer of the current sort epoch
+    bool tape = false;   // kernels with the tape's constitutive update (EMPM_ROLLOUT_TAPE)
 };
 
 static MaterialArrays sorted_material(EmpmCtx* ctx, int mc) {
@@ -796,8 +797,8 @@ static int launch_p2g_sorted(EmpmCtx* ctx, const SortedState& ss, int table, cud
     const size_t smem = sizeof(float4) * (size_t)ctx->tile_cap;
     timing_mark(ctx, 0, 0, stream);
     if (ctx->p2g_mode == 2) {
-        launch_p2g_cells(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, ctx->grid_mom, ctx->flags,
-                         uniform_material(ctx));
+        const auto launch = ss.tape ? launch_p2g_cells<true> : launch_p2g_cells<false>;
+        launch(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, ctx->grid_mom, ctx->flags, uniform_material(ctx));
     } else {
         k_p2g_tiled<<<ctx->sm_count * 2, TILE_THREADS, smem, stream>>>(t);
     }
@@ -838,8 +839,9 @@ static int launch_g2p2g_sorted(EmpmCtx* ctx, const SortedState& ss, int g2p_tabl
     const int n = ctx->n_particles;
     const TiledArgs t = sorted_args(ctx, ss, table);
     timing_mark(ctx, 6, 0, stream);
-    launch_g2p2g(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, g2p_table, ctx->grid_vel, ctx->grid_mom,
-                 ctx->flags, uniform_material(ctx));
+    const auto launch = ss.tape ? launch_g2p2g<true> : launch_g2p2g<false>;
+    launch(few_particles(ctx, n), stream, t.P, t.M, t.Fe, t.L, g2p_table, ctx->grid_vel, ctx->grid_mom, ctx->flags,
+           uniform_material(ctx));
     timing_mark(ctx, 6, 1, stream);
     CK(cudaGetLastError(), "k_g2p2g");
     return EMPM_OK;
@@ -892,8 +894,9 @@ static int launch_rollout(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, cons
         return rc;
     }
     const int n = ctx->n_particles;
+    if (!(flags & EMPM_ROLLOUT_RESUME)) ss = SortedState();
+    ss.tape = (flags & EMPM_ROLLOUT_TAPE) != 0;
     if (!(flags & EMPM_ROLLOUT_RESUME)) {
-        ss = SortedState();
         const ParticleArrays ua = particle_arrays(a, n);
         rc = launch_sort(ctx, ss, &ua, mat, stream);
         since = 0;
@@ -1009,7 +1012,7 @@ extern "C" int empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b,
     if (n_steps < 1 || n_steps > 100000) return empm_set_error(ctx, EMPM_ERR_INVALID, "n_steps %d out of [1, 100000]", n_steps);
     if (n_tables != 1 && n_tables != n_steps)
         return empm_set_error(ctx, EMPM_ERR_INVALID, "n_tables must be 1 or n_steps (%d, %d)", n_tables, n_steps);
-    if (flags & ~(EMPM_ROLLOUT_GRAPH | EMPM_ROLLOUT_RESUME | EMPM_ROLLOUT_KEEP))
+    if (flags & ~(EMPM_ROLLOUT_GRAPH | EMPM_ROLLOUT_RESUME | EMPM_ROLLOUT_KEEP | EMPM_ROLLOUT_TAPE))
         return empm_set_error(ctx, EMPM_ERR_INVALID, "unknown rollout flags %#x", flags);
     cudaStream_t s = (cudaStream_t)stream;
     const bool sorted = use_sorted(ctx);
@@ -1061,7 +1064,7 @@ extern "C" int empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b,
         key.seg_cap = ctx->seg_cap;
         key.fuse = use_fused(ctx) ? 1 : 0;
         key.params_version = ctx->params_version;
-        key.flags = flags & (EMPM_ROLLOUT_RESUME | EMPM_ROLLOUT_KEEP);
+        key.flags = flags & (EMPM_ROLLOUT_RESUME | EMPM_ROLLOUT_KEEP | EMPM_ROLLOUT_TAPE);
         if (flags & EMPM_ROLLOUT_RESUME) {
             key.start_pc = ss.pc;
             key.start_mc = ss.mc;
@@ -1247,13 +1250,9 @@ __global__ void k_debug_stress_adjoint(const float* Ft9, const float* mu, const 
     if (p >= n) return;
     M3 Ft, gF, gS;
     for (int i = 0; i < 9; ++i) { Ft.m[i] = Ft9[9 * p + i]; gF.m[i] = gF9[9 * p + i]; gS.m[i] = gS9[9 * p + i]; }
-    M3 tau;
-    SpectralGrad g;
-    switch (ms.material) {   // as the kernels of a batch of one material
-        case 0: g = constitutive_adjoint<0>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau); break;
-        case 5: g = constitutive_adjoint<5>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau); break;
-        default: g = constitutive_adjoint<-1>(Ft, mu[p], lam[p], ys[p], dt, ms, gF, gS, g_mu[p], g_lam[p], g_ys[p], tau);
-    }
+    SpectralEval e;
+    spectral_eval(Ft, mu[p], lam[p], ys[p], dt, ms, e);
+    const SpectralGrad g = spectral_adjoint(e, gF, gS, g_mu[p], g_lam[p], g_ys[p]);
     for (int i = 0; i < 9; ++i) gFt9[9 * p + i] = g.gFt.m[i];
     g_mu[p] = g.g_mu;
     g_lam[p] = g.g_lam;
@@ -1361,7 +1360,7 @@ static int launch_substep_arrays(EmpmCtx* ctx, const ParticleArrays& Pin, const 
     const int n = ctx->n_particles;
     const Launch L = make_launch(ctx, table);
     timing_mark(ctx, 0, 0, s);
-    if (warpagg) launch_p2g_cells(few_particles(ctx, n), s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags,
+    if (warpagg) launch_p2g_cells<true>(few_particles(ctx, n), s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags,
                                   uniform_material(ctx));
     else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pin, M, Fe, L, ctx->grid_mom, ctx->flags);
     timing_mark(ctx, 0, 1, s);
@@ -1449,7 +1448,7 @@ static int segment_forward(EmpmCtx* ctx, const SegmentData& d, cudaStream_t s) {
             CK(cudaMemcpyAsync(d.mats + (size_t)k * 3 * np, ab.work, 3 * np * sizeof(float), cudaMemcpyDeviceToDevice,
                                s), "snapshot");
             timing_mark(ctx, 0, 0, s);
-            if (d.sorted) launch_p2g_cells(few_particles(ctx, n), s, Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags,
+            if (d.sorted) launch_p2g_cells<true>(few_particles(ctx, n), s, Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags,
                                            uniform_material(ctx));
             else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pin, Mw, Fk, Lk, ctx->grid_mom, ctx->flags);
             timing_mark(ctx, 0, 1, s);
@@ -1514,7 +1513,7 @@ static int segment_reverse(EmpmCtx* ctx, const SegmentData& d, ParticleArrays Gp
                "restore snapshot");
             const Launch Lrec = make_launch_on(ctx, d.steps, n_steps + k);
             timing_mark(ctx, 0, 0, s);
-            if (d.sorted) launch_p2g_cells(few_particles(ctx, n), s, Pk, Mw, Fe, Lrec, ctx->grid_mom, ctx->flags,
+            if (d.sorted) launch_p2g_cells<true>(few_particles(ctx, n), s, Pk, Mw, Fe, Lrec, ctx->grid_mom, ctx->flags,
                                            uniform_material(ctx));
             else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pk, Mw, Fe, Lrec, ctx->grid_mom, ctx->flags);
             timing_mark(ctx, 0, 1, s);

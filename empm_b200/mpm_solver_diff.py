@@ -350,6 +350,10 @@ class MPMWARPDiff(object):
         launch sequence (CUDA graph when self.use_graph). Returns the state
         holding the result. `schedule` may be a (table, t_end) pair returned
         by build_schedule to replay a rollout whose schedule is already known."""
+        return self._rollout(mpm_model, state_a, state_b, dt, n_steps, step_callback, schedule)
+
+    def _rollout(self, mpm_model, state_a, state_b, dt, n_steps, step_callback=None, schedule=None, flags=0):
+        # flags: EMPM_ROLLOUT_TAPE for the forward pass of a checkpointed tape
         if n_steps <= 0:
             return state_a
         n = state_a.n_particles
@@ -363,8 +367,9 @@ class MPMWARPDiff(object):
         mat = self._material(mpm_model, state_a)
         a, b = state_a._particles(), state_b._particles()
         with torch.cuda.device(state_a.device):
-            N.check(ctx.L.empm_rollout(ctx.ptr, a, b, mat, table, n_steps, n_steps, int(self.use_graph),
-                                       _stream_ptr(state_a.device)), ctx.ptr)
+            N.check(ctx.L.empm_rollout_ex(ctx.ptr, a, b, mat, table, n_steps, n_steps,
+                                          flags | (N.ROLLOUT_GRAPH if self.use_graph else 0),
+                                          _stream_ptr(state_a.device)), ctx.ptr)
         self.time = t_end
         return state_a if n_steps % 2 == 0 else state_b
 

@@ -10,7 +10,7 @@ independent simulations at once, with continuous batching:
   particles ``[poff_i, poff_i + n_i)``.
 * Work proceeds in blocks of ``block`` substeps (fewer when every active
   request finishes sooner). Each block is one batched launch sequence
-  (``empm_rollout`` on a batch context) over every active request, each
+  (``empm_rollout_ex`` on a batch context) over every active request, each
   request on its own grid, dt and boundary conditions. A request that
   finishes inside a block is held for the rest of it (the step tables'
   ``hold`` flag: no P2G contribution, state copied through).
@@ -547,8 +547,10 @@ class GpuExecutor:
         mat = N.EmpmMaterial(self.mat["vol"][self.ai].data_ptr(), self.mat["mu"][self.ai].data_ptr(),
                              self.mat["lam"][self.ai].data_ptr(), self.mat["ys"][self.ai].data_ptr(), None,
                              self.Fe.data_ptr())
-        N.check(self.L.empm_rollout(self.ctx, views[0], views[1], mat, table, n_tables, L, 0,
-                                    self._sptr(self.fwd_stream)), self.ctx)
+        # the block's boundaries are checkpoints of the gradient requests among them
+        flags = N.ROLLOUT_TAPE if any(t.req.grad for t in active) else 0
+        N.check(self.L.empm_rollout_ex(self.ctx, views[0], views[1], mat, table, n_tables, L, flags,
+                                       self._sptr(self.fwd_stream)), self.ctx)
         if L % 2 == 1:
             self.cur = 1 - c
 

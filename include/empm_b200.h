@@ -289,12 +289,17 @@ int  empm_rollout(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMa
  *   EMPM_ROLLOUT_KEEP    leave the result in the library's sorted buffers
  *                        only: a, b and the mat arrays are not written, and a
  *                        later EMPM_ROLLOUT_RESUME call continues from it.
- * Without sorting (EMPM_OPT_SORT_EVERY 0) RESUME and KEEP have no effect.
+ *   EMPM_ROLLOUT_TAPE    the states on the way are checkpoints that will be
+ *                        differentiated: the constitutive update is the one that
+ *                        empm_segment_* and empm_adjoint_segment run, so that
+ *                        their re-runs give the same states.
+ * Without sorting (EMPM_OPT_SORT_EVERY 0) RESUME, KEEP and TAPE have no effect.
  * Graphs are cached per launch key (buffers, n_steps, options, flags, and the
  * sorted state a resumed sequence starts in), 16 at most. */
 #define EMPM_ROLLOUT_GRAPH   1
 #define EMPM_ROLLOUT_RESUME  2
 #define EMPM_ROLLOUT_KEEP    4
+#define EMPM_ROLLOUT_TAPE    8
 int  empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMaterial* mat,
                      const EmpmStep* steps, int n_tables, int n_steps, int flags, void* stream);
 
