@@ -1432,7 +1432,7 @@ def main():
     ap.add_argument("--g2p-tile", dest="g2p_tile", type=int, default=None)
     ap.add_argument("--tile-cap", dest="tile_cap", type=int, default=None)
     ap.add_argument("--seg-cap", dest="seg_cap", type=int, default=None,
-                    help="G2P adjoint: longest same-cell run per reduction (4, 8, 16, 32)")
+                    help="accepted, without effect (1, 2, 4, 8, 16, 32)")
     ap.add_argument("--fuse", dest="fuse", type=int, default=None,
                     help="1 = fused G2P + stress + P2G between cell sorts (default), 0 = separate kernels")
     ap.add_argument("--resume-blocks", dest="resume_blocks", type=int, default=None,

@@ -8,7 +8,7 @@ substeps of the caller's own workload under each candidate:
 * ``sort_every``: the period of the cell sort (8, 16, 32 substeps);
 * ``p2g_mode`` / ``tile_cap`` / ``seg_cap``: contributions summed per cell, or
   accumulation in a per-CTA shared-memory node tile of 512 / 1024 / 2048 nodes
-  (the tile shape); the longest same-cell run of the G2P adjoint, 4 or 8 lanes;
+  (the tile shape); ``seg_cap`` no longer changes a launch;
 * ``g2p_tile``: G2P gathering directly from L2 or from a staged tile;
 * ``fuse``: the G2P of each substep and the stress + P2G of the next as one
   kernel between cell sorts, or separate kernels.

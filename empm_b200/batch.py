@@ -124,7 +124,7 @@ class BatchedMPM:
         self.p2g_mode = 2
         self.g2p_tile = False
         self.tile_cap = 1024
-        self.seg_cap = 4           # G2P adjoint: longest same-cell run per reduction
+        self.seg_cap = 4           # accepted, without effect (the scatters sum whole cells)
         self.fuse = True           # fused G2P + stress + P2G between cell sorts
         self._opts = {}
         # per-instance collider lists / schedule builders

@@ -27,16 +27,11 @@
 #include "spectral.cuh"
 
 // Minimum resident CTAs (of 128 threads) per SM asked of the compiler for the
-// two particle kernels of the adjoint. The one-pass G2P adjoint keeps 18
-// accumulators live across its stencil loop: at 4 CTAs (128 registers) it
-// does not spill and took 43.5 us per 200k-particle substep, at 5 CTAs (96
-// registers, 60 B spilled) 48.0 us, at 6 (80 registers, 132 B) 45.5 us.
+// two particle kernels of the adjoint. The G2P adjoint took 35.3 us per
+// 200k-particle substep at 3 (168 registers), 38.4 at 4 and 40.6 at 5; launches
+// over few particles take CTAs of 64 threads (16k: 16.6 -> 12.6 us).
 #ifndef EMPM_ADJ_G2P_MIN_CTAS
-#define EMPM_ADJ_G2P_MIN_CTAS 4
-#endif
-// 1: the G2P adjoint's scatter loops over the outer stencil axis at run time
-#ifndef EMPM_ADJ_G2P_ROLL
-#define EMPM_ADJ_G2P_ROLL 1
+#define EMPM_ADJ_G2P_MIN_CTAS 3
 #endif
 #ifndef EMPM_ADJ_P2G_MIN_CTAS
 #define EMPM_ADJ_P2G_MIN_CTAS 4
@@ -66,7 +61,6 @@ struct AdjG2PArgs {
     float4*        gacc;   // node velocity adjoint (accumulated here)
     float4*        gx;     // out: x adjoint through G2P
     F9Planes       gFe;    // out: F_elastic adjoint
-    int            seg_cap;  // longest same-cell run summed with shuffles (a power of two)
 };
 
 // One pass over the stencil. Per node n (weight w, weight gradient dw, node
@@ -79,186 +73,153 @@ struct AdjG2PArgs {
 // with wz_k, dwz_k, (1, -2, 1) and k wz_k); the Hessian term is contracted
 // with gGv row by row.
 //
-// Lanes whose particles share an instance and base cell (contiguous in cell
-// order) sum their node-velocity adjoints with shuffles; the segment head
-// issues one reduction per node.
-// Every lane of the warp runs the node loop, invalid lanes with zeros.
-// ROUNDS < 5: runs are capped at 2^ROUNDS lanes (a.seg_cap equals it), so the
-// shuffle rounds the cap never needs are not compiled in; ROUNDS 5 takes any
-// a.seg_cap.
-template <int ROUNDS>
-__global__ void __launch_bounds__(128, EMPM_ADJ_G2P_MIN_CTAS) k_adj_g2p(const AdjG2PArgs a) {
-    const int seg_cap = ROUNDS < 5 ? (1 << ROUNDS) : a.seg_cap;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
+// The scatter is the P2G kernels' (cellsum.cuh): q_n = q0 + i Q0 + j Q1 + k Q2 and
+// the columns of gGv are the terms that a thread leaves in shared memory. Against
+// summing over the lanes of a cell with shuffles: 41.5 -> 35.3 us.
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_adj_g2p(const AdjG2PArgs a) {
+    __shared__ CellScatter<false, NT> sh;
+    cell_scatter_begin(sh);
+    const int p = blockIdx.x * NT + threadIdx.x;
     const bool live = p < a.L.n_total;
     const bool valid = live && !(a.M.sel && __ldg(a.M.sel + p) != 0);
     const int inst = live ? find_instance_particle(a.L, p) : 0;
     const StepConsts c = consts_of(a.L, inst);
     const float dt = c.step->dt;
-    const float4 xm = valid ? __ldg(a.P.x + p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const V3 x = v3(xm.x, xm.y, xm.z);
-    const Stencil st = make_stencil(x, valid ? c.inv_dx : 1.f);
-    const bool in_grid = valid && stencil_in_grid(st, c.G);
-    // segments of lanes with the same validity, instance and base cell
-    const int b0 = valid ? st.b[0] : lane, b1 = valid ? st.b[1] : -1, b2 = valid ? st.b[2] : -1;
-    const int u0 = __shfl_up_sync(0xffffffffu, b0, 1), u1 = __shfl_up_sync(0xffffffffu, b1, 1),
-              u2 = __shfl_up_sync(0xffffffffu, b2, 1);
-    const int uv = __shfl_up_sync(0xffffffffu, (int)valid, 1);
-    const int ui = __shfl_up_sync(0xffffffffu, inst, 1);
-    const bool run_head = lane == 0 || uv != (int)valid || ui != inst || u0 != b0 || u1 != b1 || u2 != b2;
-    // runs longer than seg_cap (a power of two) get another head every seg_cap
-    // lanes
-    const unsigned run_heads = __ballot_sync(0xffffffffu, run_head);
-    const int run_start = 31 - __clz(run_heads & (0xffffffffu >> (31 - lane)));
-    const bool head = run_head || ((lane - run_start) & (seg_cap - 1)) == 0;
-    const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const unsigned above = lane == 31 ? 0u : (heads & (0xffffffffu << (lane + 1)));
-    const int end = above ? (__ffs(above) - 2) : 31;
-    const int seglen = head ? end - lane + 1 : 1;
-    const int maxlen = __reduce_max_sync(0xffffffffu, seglen);
-    const unsigned take = (lane + 1 <= end ? 1u : 0u) | (lane + 2 <= end ? 2u : 0u) | (lane + 4 <= end ? 4u : 0u) |
-                          (lane + 8 <= end ? 8u : 0u) | (lane + 16 <= end ? 16u : 0u);
-
-    // x' = clamp(x + dt v'): the clamp passes the adjoint only strictly inside
-    // the band. x + dt v' lies strictly inside it exactly when the clamped x'
-    // that the forward G2P wrote does (a value clamped to a bound is not).
-    const float dx = 1.f / c.inv_dx;
-    const float lo = dx * 2.f, hi = c.grid_lim - dx * 2.f;
-    const float4 xn = valid ? __ldg(a.x_next + p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 gx4 = valid ? __ldg(a.Gn.x + p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 gv4 = valid ? __ldg(a.Gn.v + p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const V3 gxu = v3(xn.x > lo && xn.x < hi ? gx4.x : 0.f, xn.y > lo && xn.y < hi ? gx4.y : 0.f,
-                      xn.z > lo && xn.z < hi ? gx4.z : 0.f);
-    // q_n = q0 + i Q0 + j Q1 + k Q2 with Q_c = 4 inv_dx gC'[:, c]; G_c = inv_dx gGv[:, c]
-    V3 q0, Q0, Q1, Q2, G0, G1, G2;
-    {
-        const V3 gvt = v3(gv4.x, gv4.y, gv4.z) + dt * gxu;
-        const M3 gC = valid ? f9_load(a.Gn.C, p) : m3_zero();
-        const float c4 = 4.f * c.inv_dx;
-        q0 = gvt - c4 * (gC * v3(st.fx[0], st.fx[1], st.fx[2]));
-        Q0 = c4 * col(gC, 0);
-        Q1 = c4 * col(gC, 1);
-        Q2 = c4 * col(gC, 2);
-        // F' = (I + dt grad v) F_e: gGv = dt gF' F_e^T
-        const M3 gF = valid ? f9_load(a.Gn.F, p) : m3_zero();
-        const M3 gGv = (dt * c.inv_dx) * (gF * transpose(valid ? f9_load(a.Fe, p) : m3_zero()));
-        G0 = col(gGv, 0);
-        G1 = col(gGv, 1);
-        G2 = col(gGv, 2);
+    // everything the particle needs is on its way before its cell is looked at
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 xm = none, xn = none, gx4 = none, gv4 = none;
+    M3 gC = m3_zero(), gF = gC, Fe = gC;
+    if (valid) {
+        xm = __ldg(a.P.x + p);
+        xn = __ldg(a.x_next + p);
+        gx4 = __ldg(a.Gn.x + p);
+        gv4 = __ldg(a.Gn.v + p);
+        gC = f9_load(a.Gn.C, p);
+        gF = f9_load(a.Gn.F, p);
+        Fe = f9_load(a.Fe, p);
     }
-    const float wz0 = st.w[2][0], wz1 = st.w[2][1], wz2 = st.w[2][2], kz2 = 2.f * wz2;
-    const float uz0 = st.dw[2][0], uz1 = st.dw[2][1], uz2 = st.dw[2][2];
-    const V3 zero = v3(0.f, 0.f, 0.f);
-    V3 Vs = zero;                      // sum w vg (the forward's v')
-    V3 D0 = zero, D1 = zero, D2 = zero;   // columns of sum vg (x) dweight / inv_dx
-    // sum dot(vg, q) dweight + inv_dx sum H gGv^T vg, both over inv_dx (the
-    // Hessian term contracted row by row: three accumulators instead of the
-    // 18 of its moments, which let the kernel fit fewer registers)
-    V3 X3 = zero;
-    // node addresses: the block index sits above the 6 bits of the local
-    // index, so the address of node (i, j, k) is a part of its row (i, j) plus
-    // a part of k (formed once here)
-    int zpart[3];
+    const float xs[3] = {xm.x, xm.y, xm.z};
+    int b[3] = {0, 0, 0};
+    float fx[3] = {0.f, 0.f, 0.f};
+    if (valid)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int iz = st.b[2] + k;
-        zpart[k] = (iz >> 2) * 64 + (iz & 3);
-    }
-#if EMPM_ADJ_G2P_ROLL
+        for (int e = 0; e < 3; ++e) {
+            b[e] = base_node(xs[e], c.inv_dx);
+            fx[e] = base_frac(xs[e], c.inv_dx, b[e]);
+        }
+    const CellSlot cell = cell_scatter_slot(sh, valid, b, c.G, c.NB, c.boff);
+    if (valid) {
+        const bool in_grid = cell.base >= 0;
+        // x' = clamp(x + dt v'): the clamp passes the adjoint only strictly inside
+        // the band. x + dt v' lies strictly inside it exactly when the clamped x'
+        // that the forward G2P wrote does (a value clamped to a bound is not).
+        const float dx = 1.f / c.inv_dx;
+        const float lo = dx * 2.f, hi = c.grid_lim - dx * 2.f;
+        const V3 gxu = v3(xn.x > lo && xn.x < hi ? gx4.x : 0.f, xn.y > lo && xn.y < hi ? gx4.y : 0.f,
+                          xn.z > lo && xn.z < hi ? gx4.z : 0.f);
+        // q_n = q0 + i Q0 + j Q1 + k Q2 with Q_c = 4 inv_dx gC'[:, c]; G_c = inv_dx gGv[:, c]
+        V3 q0, Q0, Q1, Q2, G0, G1, G2;
+        {
+            const float c4 = 4.f * c.inv_dx;
+            const M3 Q = c4 * gC;
+            q0 = v3(gv4.x, gv4.y, gv4.z) + dt * gxu - Q * v3(fx[0], fx[1], fx[2]);
+            // F' = (I + dt grad v) F_e: gGv = dt gF' F_e^T
+            const M3 gGv = (dt * c.inv_dx) * (gF * transpose(Fe));
+            cell_scatter_put(sh, cell.slot, fx, 0.f, q0, Q);
+            cell_scatter_put(sh, cell.slot, gGv);
+            Q0 = col(Q, 0);
+            Q1 = col(Q, 1);
+            Q2 = col(Q, 2);
+            G0 = col(gGv, 0);
+            G1 = col(gGv, 1);
+            G2 = col(gGv, 2);
+        }
+        if (!in_grid) cell_scatter_edge(&sh, cell.slot, b[0], b[1], b[2], c.G, c.NB, c.boff, a.gacc, nullptr);
+        float wz[3], uz[3];
+        unsigned zpart[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            bspline_at(fx[2], k, wz[k], uz[k]);
+            zpart[k] = ((unsigned)((b[2] + k) >> 2) << 6) | ((b[2] + k) & 3);
+        }
+        const float kz2 = 2.f * wz[2], ku2 = 2.f * uz[2];
+        const V3 zero = v3(0.f, 0.f, 0.f);
+        V3 Vs = zero;                         // sum w vg (the forward's v')
+        V3 D0 = zero, D1 = zero, D2 = zero;   // columns of sum vg (x) dweight / inv_dx
+        // sum dot(vg, q) dweight + inv_dx sum H gGv^T vg, both over inv_dx (the
+        // Hessian term contracted row by row: three accumulators instead of the
+        // 18 of its moments)
+        V3 X3 = zero;
 #pragma unroll 1
-#else
+        for (int i = 0; i < 3; ++i) {
+            float wx, ux;
+            bspline_at(fx[0], i, wx, ux);
+            const float hx = bspline_d2(i);
+            const V3 qi = q0 + (float)i * Q0;
+            const int ix = b[0] + i;
+            const int xblk = c.boff + (ix >> 2) * c.NB * c.NB;
+            const unsigned xoff = (ix & 3) << 4;
+            V3 Vi = zero;
 #pragma unroll
-#endif
-    for (int i = 0; i < 3; ++i) {
-        float wx, ux;
-        bspline_at(st.fx[0], i, wx, ux);
-        const float hx = bspline_d2(i);
-        const V3 qi = q0 + (float)i * Q0;
-        V3 Vi = zero;
+            for (int j = 0; j < 3; ++j) {
+                float wy, uy;
+                bspline_at(fx[1], j, wy, uy);
+                const float wxy = wx * wy, dxy = ux * wy, xdy = wx * uy;
+                const V3 qij = j == 0 ? qi : qi + (float)j * Q1;
+                const int iy = b[1] + j;
+                const unsigned row = ((unsigned)(xblk + (iy >> 2) * c.NB) << 6) + (xoff | ((iy & 3) << 2));
+                V3 vg[3];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const float wy = st.w[1][j], uy = st.dw[1][j];
-            const float wxy = wx * wy, dxy = ux * wy, xdy = wx * uy;
-            const V3 qij = j == 0 ? qi : qi + (float)j * Q1;
-            // scatter value of node k: wz_k P + k wz_k Qr + dwz_k R
-            const V3 P = wxy * qij + dxy * G0 + xdy * G1;
-            const V3 Qr = wxy * Q2;
-            const V3 R = wxy * G2;
-            V3 vg[3];
-            float sk[3];
-            const int ix = st.b[0] + i, iy = st.b[1] + j;
-            const long long row = (long long)(c.boff + ((ix >> 2) * c.NB + (iy >> 2)) * c.NB) * 64 +
-                                  (ix & 3) * 16 + (iy & 3) * 4;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int iz = st.b[2] + k;
-                const bool node_ok = valid && (in_grid || (ix >= 0 && iy >= 0 && iz >= 0 && ix < c.G && iy < c.G &&
-                                                           iz < c.G));
-                const long long addr = node_ok ? row + zpart[k] : 0;
-                vg[k] = zero;
-                if (node_ok) {
-                    const float4 g4 = __ldg(a.vel + addr);
-                    vg[k] = v3(g4.x, g4.y, g4.z);
-                }
-                const float wz = k == 0 ? wz0 : (k == 1 ? wz1 : wz2);
-                const float uz = k == 0 ? uz0 : (k == 1 ? uz1 : uz2);
-                V3 gvg = wz * P + uz * R;
-                if (k == 1) gvg = gvg + wz1 * Qr;
-                if (k == 2) gvg = gvg + kz2 * Qr;
-                if (!node_ok) gvg = zero;
-                sk[k] = dot(vg[k], qij);
-                if (k) sk[k] += (float)k * dot(vg[k], Q2);
-                // reduction rounds unrolled, each skipped by a warp-uniform branch
-#pragma unroll
-                for (int r = 0; r < ROUNDS; ++r) {
-                    const int d = 1 << r;
-                    if (d < maxlen) {
-                        const float tx = __shfl_down_sync(0xffffffffu, gvg.x, d);
-                        const float ty = __shfl_down_sync(0xffffffffu, gvg.y, d);
-                        const float tz = __shfl_down_sync(0xffffffffu, gvg.z, d);
-                        if (take & (1u << r)) { gvg.x += tx; gvg.y += ty; gvg.z += tz; }
+                for (int k = 0; k < 3; ++k) {
+                    vg[k] = zero;
+                    if (in_grid || node_in_grid(b, i, j, k, c.G)) {
+                        const float4 g4 = __ldg(a.vel + (row + zpart[k]));
+                        vg[k] = v3(g4.x, g4.y, g4.z);
                     }
                 }
-                if (head && node_ok) red_add_v4(a.gacc + addr, make_float4(gvg.x, gvg.y, gvg.z, 0.f));
+                const V3 T0 = wz[0] * vg[0] + wz[1] * vg[1] + wz[2] * vg[2];
+                const V3 T1 = uz[0] * vg[0] + uz[1] * vg[1] + uz[2] * vg[2];
+                const V3 T2 = vg[0] - 2.f * vg[1] + vg[2];
+                // sums over the row of wz_k and dwz_k times dot(vg_k, q_ij + k Q2)
+                const float sg0 = dot(T0, qij) + dot(wz[1] * vg[1] + kz2 * vg[2], Q2);
+                const float sg1 = dot(T1, qij) + dot(uz[1] * vg[1] + ku2 * vg[2], Q2);
+                Vi = Vi + wxy * T0;
+                D0 = D0 + dxy * T0;
+                D1 = D1 + xdy * T0;
+                D2 = D2 + wxy * T1;
+                // sum_n H_n gGv^T vg_n over the row, component a = sum_b dot(G_b, H[a][b] row sum), with
+                // the pair row sums (hx wy) T0, (wx hy) T0, wxy T2, (ux uy) T0, dxy T1, xdy T1
+                const float d00 = dot(G0, T0), d10 = dot(G1, T0), d01 = dot(G0, T1), d11 = dot(G1, T1);
+                const float d21 = dot(G2, T1), d22 = dot(G2, T2);
+                const float uxy = ux * uy;
+                X3 = X3 + v3(dxy * (sg0 + d21) + (hx * wy) * d00 + uxy * d10,
+                             xdy * (sg0 + d21) + uxy * d00 + (wx * bspline_d2(j)) * d10,
+                             wxy * (sg1 + d22) + dxy * d01 + xdy * d11);
             }
-            const V3 T0 = wz0 * vg[0] + wz1 * vg[1] + wz2 * vg[2];
-            const V3 T1 = uz0 * vg[0] + uz1 * vg[1] + uz2 * vg[2];
-            const V3 T2 = vg[0] - 2.f * vg[1] + vg[2];
-            const float sg0 = wz0 * sk[0] + wz1 * sk[1] + wz2 * sk[2];
-            const float sg1 = uz0 * sk[0] + uz1 * sk[1] + uz2 * sk[2];
-            Vi = Vi + wxy * T0;
-            D0 = D0 + dxy * T0;
-            D1 = D1 + xdy * T0;
-            D2 = D2 + wxy * T1;
-            // sum_n H_n gGv^T vg_n over the row, component a = sum_b dot(G_b, H[a][b] row sum), with
-            // the pair row sums (hx wy) T0, (wx hy) T0, wxy T2, (ux uy) T0, dxy T1, xdy T1
-            const float d00 = dot(G0, T0), d10 = dot(G1, T0), d01 = dot(G0, T1), d11 = dot(G1, T1);
-            const float d21 = dot(G2, T1), d22 = dot(G2, T2);
-            const float uxy = ux * uy;
-            X3 = X3 + v3(dxy * (sg0 + d21) + (hx * wy) * d00 + uxy * d10,
-                         xdy * (sg0 + d21) + uxy * d00 + (wx * bspline_d2(j)) * d10,
-                         wxy * (sg1 + d22) + dxy * d01 + xdy * d11);
+            Vs = Vs + Vi;
         }
-        Vs = Vs + Vi;
-    }
-    if (!live) return;
-    // F' = (I + dt grad v) F_e  ->  gF_e = (I + dt grad v)^T gF' (gF' read again rather than kept live)
-    M3 A;   // I + dt grad v, grad v = inv_dx [D0 | D1 | D2] (columns)
-    {
-        const V3 dc[3] = {D0, D1, D2};
-        const float s = dt * c.inv_dx;
+        // F' = (I + dt grad v) F_e  ->  gF_e = (I + dt grad v)^T gF' (gF' read again rather than kept live)
+        M3 A;   // I + dt grad v, grad v = inv_dx [D0 | D1 | D2] (columns)
+        {
+            const V3 dc[3] = {D0, D1, D2};
+            const float s = dt * c.inv_dx;
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+            for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int cl = 0; cl < 3; ++cl) A.m[3 * r + cl] = (r == cl ? 1.f : 0.f) + s * comp(dc[cl], r);
+                for (int cl = 0; cl < 3; ++cl) A.m[3 * r + cl] = (r == cl ? 1.f : 0.f) + s * comp(dc[cl], r);
+        }
+        f9_store(a.gFe, p, transpose(A) * f9_load(a.Gn.F, p));
+        // With G = inv_dx gGv the Hessian term inv_dx^2 sum H gGv^T vg is inv_dx sum H G^T vg (in X3).
+        // The forward's C' = 4 inv_dx (...) enters the x adjoint as -4 inv_dx^2 gC'^T v' = -inv_dx (dot(Q_c, v'))_c.
+        const V3 QV = v3(dot(Q0, Vs), dot(Q1, Vs), dot(Q2, Vs));
+        const V3 gxa = gxu + c.inv_dx * (X3 - QV);
+        a.gx[p] = make_float4(gxa.x, gxa.y, gxa.z, 0.f);
+    } else if (live) {
+        f9_store(a.gFe, p, m3_zero());
+        a.gx[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    f9_store(a.gFe, p, transpose(A) * (valid ? f9_load(a.Gn.F, p) : m3_zero()));
-    // With G = inv_dx gGv the Hessian term inv_dx^2 sum H gGv^T vg is inv_dx sum H G^T vg (in X3).
-    // The forward's C' = 4 inv_dx (...) enters the x adjoint as -4 inv_dx^2 gC'^T v' = -inv_dx (dot(Q_c, v'))_c.
-    const V3 QV = v3(dot(Q0, Vs), dot(Q1, Vs), dot(Q2, Vs));
-    const V3 gxa = gxu + c.inv_dx * (X3 - QV);
-    a.gx[p] = make_float4(gxa.x, gxa.y, gxa.z, 0.f);
+    cell_scatter(sh, cell, a.gacc, nullptr);
 }
 
 // ---------------------------------------------------------------------------

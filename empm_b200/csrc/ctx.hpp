@@ -149,7 +149,7 @@ struct EmpmCtx {
     int          p2g_mode = 2;             // 0 direct reductions, 1 shared-memory tile, 2 warp-aggregated
     int          g2p_tile = 0;
     int          tile_cap = 1024;          // nodes per shared-memory tile (16 B each)
-    int          seg_cap = 4;              // warp-aggregated P2G: longest same-cell run per head
+    int          seg_cap = 4;              // accepted, without effect
     int          adj_store = 1;            // adjoint segments store substep grids instead of recomputing
     int          fuse = 1;                 // sorted rollouts fuse the G2P of one substep with the P2G of the next
     bool         fuse_ok = true;           // the uploaded step tables allow it (holds never released)

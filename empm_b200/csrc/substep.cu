@@ -1534,12 +1534,9 @@ static int segment_reverse(EmpmCtx* ctx, const SegmentData& d, ParticleArrays Gp
         ag.gacc = ab.gacc;
         ag.gx = ab.gx;
         ag.gFe = gFe;
-        ag.seg_cap = ctx->seg_cap;
         timing_mark(ctx, 3, 0, s);
-        if (ag.seg_cap == 4)
-            k_adj_g2p<2><<<blocks_for(n, 128), 128, 0, s>>>(ag);
-        else
-            k_adj_g2p<5><<<blocks_for(n, 128), 128, 0, s>>>(ag);
+        if (few_particles(ctx, n)) k_adj_g2p<64, 1><<<blocks_for(n, 64), 64, 0, s>>>(ag);
+        else k_adj_g2p<128, EMPM_ADJ_G2P_MIN_CTAS><<<blocks_for(n, 128), 128, 0, s>>>(ag);
         timing_mark(ctx, 3, 1, s);
         CK(cudaGetLastError(), "k_adj_g2p");
         AdjGridArgs gg;

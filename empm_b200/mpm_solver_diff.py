@@ -118,7 +118,7 @@ class MPMWARPDiff(object):
         self.p2g_mode = 2          # 0 direct, 1 shared-memory tile, 2 summed per cell
         self.g2p_tile = False
         self.tile_cap = 1024
-        self.seg_cap = 4           # G2P adjoint: longest same-cell run per reduction
+        self.seg_cap = 4           # accepted, without effect (the scatters sum whole cells)
         self.adj_store = True      # adjoint keeps each substep's grid and elastic F instead of recomputing
         self.fuse = True           # rollouts fuse each G2P with the next substep's stress + P2G
         self.segment_graph = True  # stored tape segments replay their substep loops from CUDA graphs

@@ -310,9 +310,8 @@ int  empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const Emp
                                     in shared memory (default) */
 #define EMPM_OPT_G2P_TILE    3   /* 1 = G2P stages the node tile in shared memory (default), 0 = direct gathers */
 #define EMPM_OPT_TILE_CAP    4   /* nodes per shared-memory tile, 27..3072 (default 1024 = 16 KiB) */
-#define EMPM_OPT_SEG_CAP     5   /* G2P adjoint: same-cell runs longer than this (a power of two, 1..32
-                                    lanes) are split, trading shuffle rounds for grid reductions
-                                    (default 4); the P2G kernels sum whole cells */
+#define EMPM_OPT_SEG_CAP     5   /* a power of two in 1..32 (default 4); accepted and without effect: the
+                                    scatters sum whole cells */
 #define EMPM_OPT_ADJ_STORE   6   /* empm_adjoint_segment: 1 = keep every substep's touched grid blocks and
                                     elastic F from the segment's forward pass for the reverse pass (default;
                                     n_steps x (2 KiB per grid block + 36 B per particle) of device memory,
