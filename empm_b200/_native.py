@@ -63,6 +63,14 @@ class EmpmStep(ctypes.Structure):
     ]
 
 
+class EmpmWindow(ctypes.Structure):
+    _fields_ = [
+        ("start", ctypes.c_float), ("end", ctypes.c_float), ("zero_until", ctypes.c_float), ("on", ctypes.c_int),
+        ("moves", ctypes.c_int), ("moved", ctypes.c_int), ("move_start", ctypes.c_double),
+        ("move_end", ctypes.c_double), ("point", F3), ("velocity", F3),
+    ]
+
+
 class EmpmParticles(ctypes.Structure):
     _fields_ = [("x", ctypes.c_void_p), ("v", ctypes.c_void_p), ("C", ctypes.c_void_p), ("F", ctypes.c_void_p)]
 
@@ -112,6 +120,8 @@ def lib():
                           ctypes.POINTER(EmpmMaterial), ctypes.POINTER(EmpmStep), P], I),
         "empm_substep_inplace": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmMaterial),
                                   ctypes.POINTER(EmpmStep), P, P], I),
+        "empm_schedule_fill": ([P, I, I, ctypes.c_double, ctypes.c_double, P, P,
+                                ctypes.POINTER(ctypes.c_double)], I),
         "empm_rollout": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmParticles),
                           ctypes.POINTER(EmpmMaterial), P, I, I, I, P], I),
         "empm_rollout_ex": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmParticles),

@@ -199,8 +199,9 @@ class CheckpointedRollout:
             new += nb.value * max(0, lengths.count(n_seg) - ctx.pooled(n_seg, block_cap))
         budget = self.store_budget
         if budget is None:
-            # segments already in the pool count as available
-            budget = torch.cuda.mem_get_info(dev)[0] // 2 + (total - new)
+            # segments already in the pool count as available; when they are all
+            # there the driver is not asked (a query waits about 2 ms)
+            budget = (torch.cuda.mem_get_info(dev)[0] // 2 if new else 0) + (total - new)
         if total > budget:
             if self.store:
                 raise MemoryError(f"storing the rollout needs {total} bytes, over the budget of {budget}")

@@ -229,11 +229,7 @@ class BatchedMPM:
         table = (N.EmpmStep * (n_steps * self.n_inst))()
         for i, sv in enumerate(self.solvers):
             sv._check_masks()
-            t = self.time
-            for s in range(n_steps):
-                sv._fill_step(table[s * self.n_inst + i], t, dt)
-                sv._modify(t, dt)
-                t = t + dt
+            sv._fill_steps(table, i, self.n_inst, self.time, dt, n_steps)
         return table, n_steps
 
     def _apply_options(self):

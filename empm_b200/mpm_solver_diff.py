@@ -297,14 +297,70 @@ class MPMWARPDiff(object):
         modify callbacks as it goes. Returns (table, t_end)."""
         self._check_masks()
         table = (N.EmpmStep * n_steps)()
+        if step_callback is None:
+            return table, self._fill_steps(table, 0, 1, t0, dt, n_steps)
         t = t0
         for s in range(n_steps):
-            if step_callback is not None:
-                step_callback(s)
+            step_callback(s)
             self._fill_step(table[s], t, dt)
             self._modify(t, dt)
             t = t + dt
         return table, t
+
+    def _fill_steps(self, table, first: int, stride: int, t, dt, n_steps: int):
+        """Fill table[first + s * stride] for n_steps substeps from solver time t,
+        running the modify callbacks in between; returns the time after the last.
+        When only the gates and points that follow their velocity differ between
+        the substeps, the library fills all but the first."""
+        windows = self._windows(t, dt) if n_steps > 1 else None
+        if windows is not None:
+            self._fill_step(table[first], t, dt)
+            t_end = N.ctypes.c_double()
+            N.check(N.lib().empm_schedule_fill(N.ctypes.byref(table, first * N.ctypes.sizeof(N.EmpmStep)), stride,
+                                               n_steps, t, dt, *windows, t_end))
+            for p, w in zip(self.collider_params, windows[0]):
+                if w.moved:
+                    p.point = tuple(w.point)
+            return t_end.value
+        for s in range(n_steps):
+            self._fill_step(table[first + s * stride], t, dt)
+            self._modify(t, dt)
+            t = t + dt
+        return t
+
+    def _windows(self, t, dt):
+        """(collider, modifier) windows for empm_schedule_fill, or None where the
+        substeps need the general path: modify callbacks other than _move_point,
+        layered releases (their threshold changes), one parameter block under two
+        registrations, and times whose arithmetic is not that of a double."""
+        colliders, modify = self.collider_params, self.modify_bc
+        mods = list(self.impulse_params) + list(self.particle_velocity_modifier_params)
+        if type(t) is not float or type(dt) is not float or not math.isfinite(t) or not math.isfinite(dt) \
+                or len(modify) != len(colliders) or len({id(p) for p in colliders}) != len(colliders) \
+                or len(colliders) > N.EMPM_MAX_COLLIDERS or len(mods) > N.EMPM_MAX_MODIFIERS:
+            return None
+        cw, mw = (N.EmpmWindow * N.EMPM_MAX_COLLIDERS)(), (N.EmpmWindow * N.EMPM_MAX_MODIFIERS)()
+        inf = math.inf
+        for w, p, mod in zip(cw, colliders, modify):
+            kind = p._kind
+            w.start, w.end, w.zero_until = -inf, inf, -inf
+            if kind != N.COLL_GRID_MASK:
+                w.start, w.end = float(_f32(p.start_time)), float(_f32(p.end_time))
+            w.on = bool(p.active) if kind in (N.COLL_GEOMETRY, N.COLL_GRID_VELOCITY) else \
+                kind in (N.COLL_SURFACE, N.COLL_CUBOID_VELOCITY, N.COLL_BOUNDING_BOX, N.COLL_GRID_MASK)
+            if kind in (N.COLL_GRID_VELOCITY, N.COLL_CUBOID_VELOCITY) and int(p.reset) == 1:
+                w.zero_until = float(_f32(p.end_time) + _f32(15.0) * _f32(dt))
+            if mod is not None:
+                if mod is not self._move_point or type(p.start_time) not in (int, float) \
+                        or type(p.end_time) not in (int, float):
+                    return None
+                w.moves, w.move_start, w.move_end = 1, p.start_time, p.end_time
+                w.point, w.velocity = N.F3(*_vec3(p.point)), N.F3(*_vec3(p.velocity))
+        for w, p in zip(mw, mods):
+            if p._kind == N.MOD_SET_VELOCITY_LAYERED:
+                return None
+            w.start, w.end, w.zero_until, w.on = float(_f32(p.start_time)), float(_f32(p.end_time)), -inf, 1
+        return cw, mw
 
     @staticmethod
     def _material(mpm_model: MPMModelStruct, mpm_state: MPMStateStruct) -> N.EmpmMaterial:

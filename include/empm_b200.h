@@ -170,6 +170,25 @@ typedef struct {
     EmpmModifier modifiers[EMPM_MAX_MODIFIERS];
 } EmpmStep;
 
+/* When one collider or modifier acts, and how it moves, over a schedule. */
+typedef struct {
+    float  start, end;     /* applies where start <= time < end (the float32 time of the substep) */
+    float  zero_until;     /* elsewhere EMPM_GATE_ZERO_ALL before this time; -inf for never */
+    int    on;             /* 0: never applies */
+    int    moves;          /* 1: point += dt * velocity after each substep in [move_start, move_end) */
+    int    moved;          /* out: 1 when it moved */
+    double move_start, move_end;   /* compared with the solver time in double */
+    float  point[3];       /* in: at the first substep; out: after the last one */
+    float  velocity[3];
+} EmpmWindow;
+
+/* Fill substeps 1..n_steps-1 of a schedule (entry s at steps[s * stride]) from
+ * its complete first entry: time, gates and moved points per substep, all else
+ * copied. Writes the gates of the first entry too and the solver time after the
+ * last substep to t_end. Host only. */
+int  empm_schedule_fill(EmpmStep* steps, int stride, int n_steps, double t0, double dt, EmpmWindow* colliders,
+                        const EmpmWindow* modifiers, double* t_end);
+
 /* Particle state buffers (device pointers, layout in the file header). */
 typedef struct {
     float* x;       /* float4 plane (x, y, z, mass) */
