@@ -77,6 +77,20 @@ struct SortedBuffers {
     size_t scan_tmp_bytes = 0;
 };
 
+// Buffers that order the particles of a single substep by cell: one block, allocated
+// on first use.
+struct OrderBuffers {
+    bool      allocated = false;
+    int       n = 0;                       // particle capacity
+    long long nb = 0;                      // block capacity
+    int2*     keys = nullptr;              // [n] cell and rank in it
+    int*      order = nullptr;             // [n] particles, those of a cell next to one another
+    int*      counts = nullptr;            // [nb * 64] particles per cell, zero between uses
+    int*      offsets = nullptr;           // [nb * 64]
+    unsigned char* marks = nullptr;        // [nb] blocks with particles, zero between uses
+    int*      next = nullptr;
+};
+
 // Buffers of the reverse-mode path (empm_adjoint_segment), allocated on first use.
 struct AdjointBuffers {
     int     capacity = 0;      // substeps per segment the buffers hold
@@ -154,6 +168,7 @@ struct EmpmCtx {
     int          fuse = 1;                 // sorted rollouts fuse the G2P of one substep with the P2G of the next
     bool         fuse_ok = true;           // the uploaded step tables allow it (holds never released)
     SortedBuffers sb;
+    OrderBuffers ob;
     AdjointBuffers adj;
     // per-kernel event timing (stream path only)
     bool         timing = false;

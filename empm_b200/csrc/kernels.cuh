@@ -574,14 +574,9 @@ __global__ void __launch_bounds__(128, EMPM_G2P_MIN_CTAS) k_g2p_direct(ParticleA
 // Sort key of a particle: its base cell in block-major order over the whole
 // batch, ((boff + block) << 6) | in-block cell, so one counting sort orders
 // particles by instance, 4^3 block and cell. Out-of-band cells are clamped.
-__global__ void k_sort_keys(const float4* x, Launch L, int* keys, int* ranks, int* cell_counts, int* block_counts) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= L.n_total) return;
-    const int inst = find_instance_particle(L, p);
-    const InstanceConsts* I = L.inst + inst;
+__device__ __forceinline__ int cell_key(const InstanceConsts* I, float4 xm) {
     const int G = __ldg(&I->G), NB = __ldg(&I->NB);
     const float inv_dx = __ldg(&I->inv_dx);
-    const float4 xm = __ldg(x + p);
     const float xs[3] = {xm.x, xm.y, xm.z};
     int b[3];
 #pragma unroll
@@ -590,7 +585,14 @@ __global__ void k_sort_keys(const float4* x, Launch L, int* keys, int* ranks, in
         b[a] = t < 0 ? 0 : (t >= G ? G - 1 : t);
     }
     const int blk = __ldg(&I->boff) + block_of(b[0], b[1], b[2], NB);
-    const int key = (blk << 6) | ((b[0] & 3) << 4) | ((b[1] & 3) << 2) | (b[2] & 3);
+    return (blk << 6) | ((b[0] & 3) << 4) | ((b[1] & 3) << 2) | (b[2] & 3);
+}
+
+__global__ void k_sort_keys(const float4* x, Launch L, int* keys, int* ranks, int* cell_counts, int* block_counts) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= L.n_total) return;
+    const int key = cell_key(L.inst + find_instance_particle(L, p), __ldg(x + p));
+    const int blk = key >> 6;
     keys[p] = key;
     ranks[p] = atomicAdd(cell_counts + key, 1);
     atomicAdd(block_counts + blk, 1);
@@ -633,6 +635,53 @@ __global__ void k_cell_scan(int* cell_counts, int* block_counts, const int* bloc
     for (int k = lane; k * chunk < cnt; k += 32) chunks[co + k] = make_int2(off + k * chunk, min(chunk, cnt - k * chunk));
     __syncwarp();
     if (lane == 0) block_counts[warp] = 0;
+}
+
+// -------------------------------------------------------------------------
+// single substeps of many particles: the order of the cells
+// -------------------------------------------------------------------------
+// Puts the particles of a cell next to one another for one P2G, without moving
+// their state: counts and ranks per cell, a range of the order per cell (cells come
+// in any order, so a block's cells claim theirs with one atomic instead of a scan
+// over the grid), the particles into the ranges. 500k particles in random order,
+// 128^3 cells: 12.3 + 4.8 + 6.6 us; the first is bound by its returning atomics (43.7
+// us while every particle marked its block, now the first of each cell does).
+__global__ void k_order_count(const float4* x, Launch L, int2* keys, int* counts, unsigned char* marks, int* next) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) *next = 0;
+    if (p >= L.n_total) return;
+    const InstanceConsts* I = L.inst + find_instance_particle(L, p);
+    const int key = cell_key(I, __ldg(x + p));
+    const int rank = atomicAdd(counts + key, 1);
+    if (rank == 0) marks[key >> 6] = 1;
+    keys[p] = make_int2(key, rank);
+}
+
+__global__ void __launch_bounds__(256) k_order_ranges(Launch L, int* counts, int* offsets, unsigned char* marks,
+                                                      int* next) {
+    const int lane = threadIdx.x & 31;
+    for_touched_blocks(marks, L, true, [&](int b) {
+        const long long c0 = ((long long)b << 6) + 2 * lane;
+        const int2 n = *reinterpret_cast<const int2*>(counts + c0);
+        int incl = n.x + n.y;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        int base = 0;
+        if (lane == 31) base = atomicAdd(next, incl);
+        const int first = __shfl_sync(0xffffffffu, base, 31) + incl - n.x - n.y;
+        *reinterpret_cast<int2*>(offsets + c0) = make_int2(first, first + n.x);
+        *reinterpret_cast<int2*>(counts + c0) = make_int2(0, 0);
+    });
+}
+
+__global__ void k_order_fill(const int2* keys, const int* offsets, int* order, int n) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int2 k = __ldg(keys + p);
+    order[__ldg(offsets + k.x) + k.y] = p;
 }
 
 struct PermuteArgs {
@@ -738,16 +787,21 @@ __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid,
     cell_scatter(sh, cell, grid, flags);
 }
 
+// order: NULL for particles sorted by cell, else the order that makes them so (single
+// substeps, k_order_*). Reading the state through it costs 15 sectors a particle: 500k
+// in random order 71.9 us (jelly), 82.6 (sand), against 42 us sorted.
 template <int NT, int MAT, int MINB, bool TAPE>
 __global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
-                                                        float4* grid, unsigned char* flags) {
+                                                        float4* grid, unsigned char* flags, const int* order) {
     __shared__ CellScatter<true, NT> sh;
     cell_scatter_begin(sh);
-    const int p = blockIdx.x * NT + threadIdx.x;
-    const StepConsts c = consts_of(L, p < L.n_total ? find_instance_particle(L, p) : 0);
+    int p = blockIdx.x * NT + threadIdx.x;
+    const bool in_range = p < L.n_total;
+    if (order && in_range) p = __ldg(order + p);
+    const StepConsts c = consts_of(L, in_range ? find_instance_particle(L, p) : 0);
     const EmpmStep& sp = *c.step;
     // a held instance contributes nothing this substep
-    const bool valid = p < L.n_total && !(M.sel && __ldg(M.sel + p) != 0) && !sp.hold;
+    const bool valid = in_range && !(M.sel && __ldg(M.sel + p) != 0) && !sp.hold;
     float4 xm = make_float4(0.f, 0.f, 0.f, 0.f), vv = xm;
     M3 C = m3_zero(), F = C;
     float mu = 0.f, lam = 0.f, ys = 0.f, vol = 0.f;
@@ -907,8 +961,8 @@ static inline void launch_g2p2g(bool few, cudaStream_t s, const ParticleArrays& 
 template <bool TAPE>
 static inline void launch_p2g_cells(bool few, cudaStream_t s, const ParticleArrays& P, const MaterialArrays& M,
                                     const F9Planes& Fe, const Launch& L, float4* mom, unsigned char* flags,
-                                    int material) {
-    EMPM_CELL_LAUNCH(k_p2g_cells, EMPM_P2G_MIN_CTAS, TAPE, L.n_total, few, material, s, P, M, Fe, L, mom, flags);
+                                    int material, const int* order = nullptr) {
+    EMPM_CELL_LAUNCH(k_p2g_cells, EMPM_P2G_MIN_CTAS, TAPE, L.n_total, few, material, s, P, M, Fe, L, mom, flags, order);
 }
 
 // -------------------------------------------------------------------------
