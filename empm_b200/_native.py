@@ -75,6 +75,11 @@ class EmpmParticles(ctypes.Structure):
     _fields_ = [("x", ctypes.c_void_p), ("v", ctypes.c_void_p), ("C", ctypes.c_void_p), ("F", ctypes.c_void_p)]
 
 
+class EmpmInstanceArrays(ctypes.Structure):
+    _fields_ = [(k, ctypes.c_void_p) for k in ("x", "v", "vol", "density", "E", "nu", "yield_stress")] + [
+        (k, ctypes.c_int) for k in ("first", "count", "broadcast", "reserved")]
+
+
 class EmpmMaterial(ctypes.Structure):
     _fields_ = [
         ("vol", ctypes.c_void_p), ("mu", ctypes.c_void_p), ("lam", ctypes.c_void_p),
@@ -120,6 +125,7 @@ def lib():
                           ctypes.POINTER(EmpmMaterial), ctypes.POINTER(EmpmStep), P], I),
         "empm_substep_inplace": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmMaterial),
                                   ctypes.POINTER(EmpmStep), P, P], I),
+        "empm_load_instances": ([P, I, I, I, ctypes.POINTER(EmpmParticles), P, P, P, P, P, P], I),
         "empm_schedule_fill": ([P, I, I, ctypes.c_double, ctypes.c_double, P, P,
                                 ctypes.POINTER(ctypes.c_double)], I),
         "empm_rollout": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmParticles),

@@ -151,34 +151,51 @@ class BatchedMPM:
     def load_state(self, instances: Optional[Sequence[int]] = None):
         """(Re)load positions, velocities and materials of the given instances
         (all by default) from their specs; C = 0, F = I."""
-        idx = range(self.n_inst) if instances is None else instances
+        idx = list(range(self.n_inst) if instances is None else instances)
         dev = self.device
-        b = self.cur
-        for i in idx:
-            s = self.specs[i]
-            sl = self._sl(i)
-            t = lambda a: torch.as_tensor(np.ascontiguousarray(a), dtype=DTYPE).to(dev, non_blocking=True)  # noqa
-            self._x4[b][sl, :3] = t(s.x)
-            self._v4[b][sl, :3] = t(s.v) if s.v is not None else 0.0
-            self._v4[b][sl, 3] = 0.0
-            self.vol[sl] = t(s.vol)
-            self.density[sl] = t(s.rho)
-            self.E[sl] = t(s.E)
-            self.nu[sl] = t(s.nu)
-            self.yield_stress[sl] = t(s.yield_stress) if s.yield_stress is not None else 0.0
-        # C = 0 and F = I for the whole batch (per-instance planes are strided)
-        if instances is None:
-            self._C[b].zero_()
-            _f9_identity(self._F[b], self.n)
-        else:
-            C = _f9_unpack(self._C[b], self.n).clone()
-            F = _f9_unpack(self._F[b], self.n).clone()
-            for i in idx:
-                sl = self._sl(i)
-                C[sl] = 0.0
-                F[sl] = torch.eye(3, device=dev)
-            _f9_pack(self._C[b], C)
-            _f9_pack(self._F[b], F)
+        table = (N.EmpmInstanceArrays * len(idx))()
+        arrays = {}     # an array that several instances share goes up once per call
+        for e, i in zip(table, idx):
+            s, n = self.specs[i], self.counts[i]
+            e.first, e.count = int(self.poff[i]), n
+            for bit, (name, a) in enumerate((("x", s.x), ("v", s.v), ("vol", s.vol), ("density", s.rho), ("E", s.E),
+                                             ("nu", s.nu), ("yield_stress", s.yield_stress))):
+                if a is None and name in ("v", "yield_stress"):
+                    continue
+                key = (id(a), n, bit < 2)
+                if key not in arrays:
+                    arrays[key] = (a, *_host_rows(a, (n, 3) if bit < 2 else (n,)), [])
+                e.broadcast |= arrays[key][2] << bit
+                arrays[key][3].append((e, name))
+        # small arrays and the table travel together, one copy instead of one each;
+        # from 256 KB on gathering them on the host would cost more than their copies
+        at = ctypes.sizeof(table)
+        packed = []
+        for key, (_, host, _, users) in arrays.items():
+            nbytes = host.numel() * 4
+            if nbytes < 256 << 10:
+                packed.append((at, host, users))
+                at += nbytes
+        staging = torch.empty(at, dtype=torch.uint8, device=dev)
+        for off, _, users in packed:
+            for e, name in users:
+                setattr(e, name, staging.data_ptr() + off)
+        live = [staging]
+        for _, host, _, users in arrays.values():
+            if host.numel() * 4 >= 256 << 10:
+                live.append(host.to(dev, non_blocking=True))
+                for e, name in users:
+                    setattr(e, name, live[-1].data_ptr())
+        buf = np.empty(at, np.uint8)
+        buf[:ctypes.sizeof(table)] = np.frombuffer(table, np.uint8)
+        for off, host, _ in packed:
+            buf[off:off + 4 * host.numel()].view(np.float32)[:] = host.reshape(-1).numpy()
+        staging.copy_(torch.from_numpy(buf))
+        with torch.cuda.device(dev):
+            N.check(self.L.empm_load_instances(staging.data_ptr(), len(idx), max((self.counts[i] for i in idx), default=0),
+                                               self.n, self._views(self.cur), self.vol.data_ptr(),
+                                               self.density.data_ptr(), self.E.data_ptr(), self.nu.data_ptr(),
+                                               self.yield_stress.data_ptr(), _stream_ptr(dev)))
         self.prepare()
 
     def prepare(self):
@@ -287,6 +304,20 @@ class BatchedMPM:
                 self.ptr = None
         except Exception:
             pass
+
+
+def _host_rows(a, shape):
+    """(contiguous float32 host tensor, broadcast): the rows of a that a tensor of
+    `shape` takes from it, or one row for all."""
+    t = torch.as_tensor(np.ascontiguousarray(a), dtype=DTYPE)
+    while t.dim() > len(shape) and t.shape[0] == 1:
+        t = t[0]
+    if tuple(t.shape) == shape:
+        return t.contiguous(), 0
+    row = t[0] if t.dim() == len(shape) and t.shape[0] == 1 else t
+    if tuple(row.shape) == shape[1:]:
+        return row.contiguous(), 1
+    return t.expand(shape).contiguous(), 0
 
 
 def block_flags(done: int, k: int, n_steps: int, use_graph: bool, resume: bool) -> int:

@@ -23,9 +23,18 @@ from . import _native as N
 from .mpm_data_structure import _stream_ptr
 
 
-def _offsets(counts: Sequence[int], device) -> Tuple[Tensor, int]:
-    off = np.concatenate([[0], np.cumsum(np.asarray(counts, dtype=np.int64))]).astype(np.int32)
-    return torch.as_tensor(off, device=device), int(max(counts) if len(counts) else 0)
+def _pair_tables(x_counts, y_counts, device):
+    """Row offsets (int32) and sizes (float, at least 1) of the pairs' clouds on the
+    device, in one copy: x_off, y_off, nx, ny."""
+    n = len(x_counts)
+    host = np.zeros(4 * n + 2, np.int32)
+    for k, counts in enumerate((x_counts, y_counts)):
+        counts = np.asarray(counts, dtype=np.int64)
+        host[k * (n + 1) + 1:(k + 1) * (n + 1)] = np.cumsum(counts)
+        host[2 * n + 2 + k * n:2 * n + 2 + (k + 1) * n] = np.maximum(counts, 1).astype(np.float32).view(np.int32)
+    dev = torch.from_numpy(host).to(device)
+    sizes = dev[2 * n + 2:].view(torch.float32)
+    return dev[:n + 1], dev[n + 1:2 * n + 2], sizes[:n], sizes[n:]
 
 
 class _ChamferPairs(torch.autograd.Function):
@@ -35,8 +44,8 @@ class _ChamferPairs(torch.autograd.Function):
         x = x.detach().float().contiguous()
         y = y.detach().float().contiguous().to(dev)
         n_pairs = len(x_counts)
-        x_off, max_nx = _offsets(x_counts, dev)
-        y_off, max_ny = _offsets(y_counts, dev)
+        x_off, y_off, nx, ny = _pair_tables(x_counts, y_counts, dev)
+        max_nx, max_ny = max(x_counts), max(y_counts)
         s_xy = torch.empty(n_pairs, dtype=torch.float32, device=dev)
         s_yx = torch.empty_like(s_xy)
         nn_x = torch.empty(x.shape[0], dtype=torch.int32, device=dev)
@@ -48,8 +57,6 @@ class _ChamferPairs(torch.autograd.Function):
                                            y_off.data_ptr(), y.shape[0], max_ny, n_pairs, s_xy.data_ptr(),
                                            s_yx.data_ptr(), nn_x.data_ptr(), nn_y.data_ptr(), work.data_ptr(),
                                            nb.value, _stream_ptr(dev)))
-        nx = torch.as_tensor(np.maximum(np.asarray(x_counts), 1), dtype=torch.float32, device=dev)
-        ny = torch.as_tensor(np.maximum(np.asarray(y_counts), 1), dtype=torch.float32, device=dev)
         ctx.save_for_backward(x, y, x_off, y_off, nn_x, nn_y, nx, ny)
         return s_xy / nx + s_yx / ny
 

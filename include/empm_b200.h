@@ -322,6 +322,24 @@ int  empm_rollout(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMa
 int  empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMaterial* mat,
                      const EmpmStep* steps, int n_tables, int n_steps, int flags, void* stream);
 
+/* Device arrays of one instance for empm_load_instances; v and yield_stress may be
+ * NULL (zeros). Bit k of broadcast: the k-th array (in this order) has one row for
+ * all particles. */
+typedef struct {
+    const float *x, *v;                        /* [count, 3] */
+    const float *vol, *density, *E, *nu, *yield_stress;   /* [count] */
+    int first, count;                          /* rows of the batch */
+    int broadcast;
+    int reserved;                              /* 0 */
+} EmpmInstanceArrays;
+
+/* State and material rows of the listed instances from their arrays, C = 0 and F = I
+ * (the mass lane of x is left to empm_prepare). table: device array; max_count: the
+ * largest count in it; n_total: rows of the batch's planes. */
+int  empm_load_instances(const EmpmInstanceArrays* table, int n_instances, int max_count, int n_total,
+                         EmpmParticles* out, float* vol, float* density, float* E, float* nu, float* yield_stress,
+                         void* stream);
+
 /* Launch options of a context (empm_ctx_set_option). */
 #define EMPM_OPT_SORT_EVERY  1   /* rollouts re-sort particles by 4^3 cell block every N substeps; 0 = no sorting (default 32) */
 #define EMPM_OPT_P2G_MODE    2   /* sorted-path P2G: 0 = one 16-byte reduction per particle and node,
