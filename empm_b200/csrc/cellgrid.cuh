@@ -24,11 +24,12 @@
 
 namespace empm {
 
-// Squared distance, one rounding per product and sum pair, spelled out so that
-// every search forms it alike.
+// Squared distance, spelled out so that every search forms it alike: the order in
+// which the compiler contracts dx * dx + dy * dy + dz * dz, which decides between
+// neighbours whose distances differ in the last bit.
 __device__ __forceinline__ float point_dist2(float qx, float qy, float qz, float px, float py, float pz) {
     const float dx = qx - px, dy = qy - py, dz = qz - pz;
-    return __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+    return __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
 }
 
 struct SetGrid {

@@ -100,3 +100,22 @@ def test_chamfer_cells_equal_brute_force(kind, sizes):
     assert torch.equal(res[0][1], res[1][1]) and torch.equal(res[0][2], res[1][2])
     n = torch.as_tensor([xc, yc], dtype=torch.float64)
     assert ((res[0][0] - res[1][0]).abs() <= 2 * n * 2.0 ** -24 * res[0][0] + 1e-30).all()
+
+
+@pytest.mark.parametrize("n", [600, 1500])           # the brute-force search, the cell grid
+def test_last_bit_of_the_distance_decides(n):
+    """Pairs of points at equal true distance, (a, b, c) and (b, a, c) off their
+    query: their order is that of dz^2 + (dx^2 + rounded dy^2), each sum rounded
+    once. Offsets are multiples of 2^-16, so differences are exact in float32 and
+    the sums before rounding in float64."""
+    rng = np.random.default_rng(3)
+    q = 8.0 * np.stack(np.unravel_index(np.arange(n), (12, 12, 12)), 1)
+    o = rng.integers(1000, 60000, (n, 3)) / 65536.0
+    pts = np.stack([q - o, q - o[:, [1, 0, 2]]], 1).reshape(-1, 3)
+    f32 = lambda a: a.astype(np.float32).astype(np.float64)  # noqa: E731
+    dist = [f32(d[:, 2] ** 2 + f32(d[:, 0] ** 2 + f32(d[:, 1] ** 2))) for d in (o, o[:, [1, 0, 2]])]
+    assert (dist[0] != dist[1]).sum() > n // 10
+    want = np.where((dist[1] < dist[0])[:, None], [1, 0], [0, 1]) + 2 * np.arange(n)[:, None]
+    t = lambda a: torch.as_tensor(a.astype(np.float32), device=DEV)  # noqa: E731
+    idx, _ = _search("brute" if n < 1000 else "cells", t(q), t(pts), 2, False)
+    assert np.array_equal(idx.cpu().numpy(), want)
