@@ -126,6 +126,7 @@ def lib():
         "empm_substep_inplace": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmMaterial),
                                   ctypes.POINTER(EmpmStep), P, P], I),
         "empm_load_instances": ([P, I, I, I, ctypes.POINTER(EmpmParticles), P, P, P, P, P, P], I),
+        "empm_matrix_rows": ([P, I, P, P], I),
         "empm_schedule_fill": ([P, I, I, ctypes.c_double, ctypes.c_double, P, P,
                                 ctypes.POINTER(ctypes.c_double)], I),
         "empm_rollout": ([P, ctypes.POINTER(EmpmParticles), ctypes.POINTER(EmpmParticles),

@@ -47,6 +47,12 @@ def _f9_pack(dst: Tensor, m: Tensor) -> None:
 
 
 def _f9_unpack(src: Tensor, n: int) -> Tensor:
+    if n > 0 and type(src) is Tensor and src.is_cuda and src.dtype == DTYPE and not src.requires_grad \
+            and src.is_contiguous() and src.numel() >= 9 * n and src.data_ptr() % 16 == 0:
+        out = torch.empty((n, 3, 3), dtype=DTYPE, device=src.device)
+        with torch.cuda.device(src.device):
+            N.check(N.lib().empm_matrix_rows(src.data_ptr(), n, out.data_ptr(), _stream_ptr(src.device)))
+        return out
     return torch.cat([src[: 4 * n].view(n, 4), src[4 * n: 8 * n].view(n, 4), src[8 * n: 9 * n].view(n, 1)],
                      dim=1).view(n, 3, 3)
 

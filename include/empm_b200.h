@@ -322,6 +322,9 @@ int  empm_rollout(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMa
 int  empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b, const EmpmMaterial* mat,
                      const EmpmStep* steps, int n_tables, int n_steps, int flags, void* stream);
 
+/* The n matrices of f9 planes as rows of 9 floats (both 16-byte aligned). */
+int  empm_matrix_rows(const float* planes, int n, float* out, void* stream);
+
 /* Device arrays of one instance for empm_load_instances; v and yield_stress may be
  * NULL (zeros). Bit k of broadcast: the k-th array (in this order) has one row for
  * all particles. */
