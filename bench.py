@@ -58,7 +58,7 @@ def load_peaks():
 # particle count on a B200: (workload, kernel, particles) -> bytes per launch.
 NCU_DRAM_BYTES = {
     ("c4", "stress_p2g", 3172508): 403.197184e6 + 110.350592e6,
-    ("c4", "g2p2g", 3172508): 248.482048e6 + 127.045632e6,
+    ("c4", "g2p2g", 3172508): 248.531456e6 + 119.240448e6,
     ("c3", "adj_p2g", 200000): 38.966272e6 + 0.203008e6,
     ("lbs", "blend", 2000000): 196.818688e6 + 41.4976e6,
 }
@@ -115,6 +115,12 @@ def rollout_launches(n_steps: int, block: int, sort_every: int, resume: bool, fu
             unsorts += 1
         done += k
     return 2 * n_steps + particle + 4 * sorts + unsorts
+
+
+def kernel_launches(n_steps: int, block: int, sort_every: int, resume: bool, fused: bool = True) -> int:
+    """rollout_launches without the touched-block list, which the grid update
+    no longer needs: one launch less per substep."""
+    return rollout_launches(n_steps, block, sort_every, resume, fused) - n_steps
 
 
 def bytes_per_particle(material: str):
@@ -449,7 +455,7 @@ def run_ours(args):
                                f"rollout in this run ({stream_ms:.2f} ms vs {ms / args.steps:.2f} ms graph)"},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": METRIC, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "gpu_launches": rollout_launches(w.T, w.T, solver.sort_every, False, dom == "g2p2g") * args.steps,
+        "gpu_launches": kernel_launches(w.T, w.T, solver.sort_every, False, dom == "g2p2g") * args.steps,
         "clocks": clk,
     }
     print(json.dumps(line), flush=True)
@@ -752,7 +758,7 @@ def run_ours_c4(args):
                                f"population rollout in this run ({stream_ms:.2f} ms vs {ms / args.steps:.2f} ms graph)"},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": METRIC, "h2d_bytes_per_step": total * 36, "d2h_bytes_per_step": total * 12},
-        "gpu_launches": rollout_launches(T, 50, bopts["sort_every"], resume, dom == "g2p2g") * args.steps,
+        "gpu_launches": kernel_launches(T, 50, bopts["sort_every"], resume, dom == "g2p2g") * args.steps,
         "clocks": clk,
     }
     print(json.dumps(line), flush=True)
@@ -965,10 +971,10 @@ def run_ours_c3(args):
         "e2e": {"value": e2e_value, "unit": METRIC, "h2d_bytes_per_step": n * (12 + 12 + 4 + 4),
                 "d2h_bytes_per_step": n * 12 + 12,
                 "path": "MPMDifferentiableSimulation.apply + loss.backward() with pinned host inputs"},
-        # per substep, not counting the cell sorts and permutations: with stored segments the forward's 4 (P2G,
-        # block list, grid update writing the store, G2P) and the reverse pass's 4 (grid restore, the 3 adjoint
-        # kernels); with checkpoints also the plain forward's 4 before them
-        "gpu_launches": (8 if stored[-1] else 12) * w.T * args.steps,
+        # per substep, not counting the cell sorts, permutations and segment ends: with stored segments the
+        # forward's 2 (fused kernel, grid update writing the store) and the reverse pass's 3 adjoint kernels;
+        # with checkpoints also the plain forward's 2 before them
+        "gpu_launches": (5 if stored[-1] else 7) * w.T * args.steps,
         "clocks": clk,
     }
     print(json.dumps(line), flush=True)
@@ -1193,10 +1199,10 @@ def measure_c5(args, dev, world, rank, local, cpu_baseline_leg=True):
         "e2e": {"value": value, "unit": METRIC, "h2d_bytes_per_step": h2d[0], "d2h_bytes_per_step":
                 sum(r[2] * (24 if not r[1] else 24) for r in ok),
                 "path": "MPMServer.submit with host (numpy) requests -> results on the host"},
-        # 4 per forward substep of a block (P2G, block list, grid update, G2P) and 8 per substep of a
-        # gradient request's adjoint (its segment re-run and reverse pass); cell sorts and write-backs
+        # 2 per forward substep of a block (fused kernel, grid update) and 5 per substep of a gradient
+        # request's adjoint (its segment re-run and reverse pass); cell sorts, block ends and write-backs
         # are not counted
-        "gpu_launches": 4 * stats["substeps"] + 8 * n_grad_substeps,
+        "gpu_launches": 2 * stats["substeps"] + 5 * n_grad_substeps,
         "clocks": clk,
     }
     return line

@@ -9,9 +9,9 @@
 // point. Queries run in cell order as well, so that the lanes of a warp visit the
 // same cells together.
 //
-// 500k queries among 50k points, k = 16: 0.66 ms for the search (0.77 with the k best in
-// local memory) and 0.05 ms for the sorting, bound by the insertions of candidates, which one lane or another of a
-// warp makes for nearly every point it looks at.
+// 500k queries among 50k points, k = 16: 0.66 ms for the search (0.77 with the k best
+// in local memory) and 0.05 ms for the sorting, bound by the insertions of candidates,
+// which one lane or another of a warp makes for nearly every point it looks at.
 //
 // Results are those of the brute-force search bit for bit: the same distance
 // expression, ties in index order, and points or queries that are not finite have

@@ -1434,11 +1434,11 @@ static int ensure_adjoint_buffers(EmpmCtx* ctx, int n_steps) {
 
 // One forward substep on explicit particle arrays (the states of a segment).
 static int launch_substep_arrays(EmpmCtx* ctx, const ParticleArrays& Pin, const ParticleArrays& Pout,
-                                 const MaterialArrays& M, F9Planes Fe, int table, bool warpagg, cudaStream_t s) {
+                                 const MaterialArrays& M, F9Planes Fe, int table, bool cells, cudaStream_t s) {
     const int n = ctx->n_particles;
     const Launch L = make_launch(ctx, table);
     timing_mark(ctx, 0, 0, s);
-    if (warpagg) launch_p2g_cells<true>(few_particles(ctx, n), s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags,
+    if (cells) launch_p2g_cells<true>(few_particles(ctx, n), s, Pin, M, Fe, L, ctx->grid_mom, ctx->flags,
                                   uniform_material(ctx));
     else k_p2g_direct<<<blocks_for(n, 128), 128, 0, s>>>(Pin, M, Fe, L, ctx->grid_mom, ctx->flags);
     timing_mark(ctx, 0, 1, s);
