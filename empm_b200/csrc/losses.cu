@@ -26,17 +26,20 @@ constexpr int kThreads = 256;
 inline int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / threads); }
 
 // For every query point q of pair blockIdx.y: nearest point of the pair's
-// target set, its squared distance added to sum[pair].
+// target set, its squared distance added to sum[pair]. rest: only the pair's first
+// rest[pair] of the queries rest_row.
 __global__ void __launch_bounds__(kThreads) k_nn(const float* __restrict__ q, const int* __restrict__ q_off,
                                                  const float* __restrict__ t, const int* __restrict__ t_off,
-                                                 int* __restrict__ nn, float* __restrict__ sum) {
+                                                 int* __restrict__ nn, float* __restrict__ sum,
+                                                 const int* __restrict__ rest, const int* __restrict__ rest_row) {
     __shared__ float4 tile[kThreads];
     const int pair = blockIdx.y;
-    const int q0 = __ldg(q_off + pair), q1 = __ldg(q_off + pair + 1);
+    const int q0 = __ldg(q_off + pair), q1 = rest ? q0 + __ldg(rest + pair) : __ldg(q_off + pair + 1);
     const int t0 = __ldg(t_off + pair), t1 = __ldg(t_off + pair + 1);
-    const int i = q0 + blockIdx.x * kThreads + threadIdx.x;
+    const int slot = q0 + blockIdx.x * kThreads + threadIdx.x;
     if (q0 + (int)(blockIdx.x * kThreads) >= q1) return;   // whole CTA beyond this pair's queries
-    const bool live = i < q1;
+    const bool live = slot < q1;
+    const int i = live && rest ? __ldg(rest_row + slot) : slot;
     float qx = 0.f, qy = 0.f, qz = 0.f;
     if (live) { qx = __ldg(q + 3 * i); qy = __ldg(q + 3 * i + 1); qz = __ldg(q + 3 * i + 2); }
     float best = FLT_MAX;
@@ -81,9 +84,15 @@ __global__ void __launch_bounds__(kThreads) k_nn_cells(const PointSets P, const 
         const float4 q = __ldg(w.sorted + t);
         Nearest<1> best;
         best.clear(FLT_MAX);
-        nearest_search<1>(w.grids[in_a ? P.sets_a + pair : pair], w.start, w.sorted, q.x, q.y, q.z, 1, -1, 1, best);
-        (in_a ? nn_x : nn_y)[__float_as_int(q.w)] = best.i[0];
-        if (best.i[0] >= 0) v = best.d[0];
+        const int* off = in_a ? P.b_off : P.a_off;
+        if (nearest_search<1>(w.grids[in_a ? P.sets_a + pair : pair], w.start, w.sorted, q.x, q.y, q.z, 1, -1,
+                              __ldg(off + pair + 1) - __ldg(off + pair), best)) {
+            (in_a ? nn_x : nn_y)[__float_as_int(q.w)] = best.i[0];
+            if (best.i[0] >= 0) v = best.d[0];
+        } else {
+            const int first = in_a ? __ldg(P.a_off + pair) : P.rows_a + __ldg(P.b_off + pair);
+            w.rest_row[first + atomicAdd(w.rest + set, 1)] = __float_as_int(q.w);
+        }
     }
     // one atomic per block, or per thread where two clouds meet in it
     if (threadIdx.x == 0) ends[0] = set;
@@ -151,6 +160,24 @@ __global__ void k_pair_index(const int* off, int n_pairs, int* pair_of, int n) {
         if (_rc != EMPM_OK) return _rc;                                          \
     } while (0)
 
+// The brute-force search both ways. rest: only the queries left over by the cells
+// (counts of the x clouds, then of the y clouds).
+static int launch_nn(const float* x, const int* x_off, int max_nx, const float* y, const int* y_off, int max_ny,
+                     int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y, const int* rest,
+                     const int* rest_x, const int* rest_y, cudaStream_t s) {
+    if (max_nx > 0) {
+        k_nn<<<dim3(blocks_for(max_nx, kThreads), n_pairs), kThreads, 0, s>>>(x, x_off, y, y_off, nn_x, sum_xy, rest,
+                                                                             rest_x);
+        CKL(cudaGetLastError(), "k_nn (x -> y)");
+    }
+    if (max_ny > 0) {
+        k_nn<<<dim3(blocks_for(max_ny, kThreads), n_pairs), kThreads, 0, s>>>(y, y_off, x, x_off, nn_y, sum_yx,
+                                                                             rest ? rest + n_pairs : nullptr, rest_y);
+        CKL(cudaGetLastError(), "k_nn (y -> x)");
+    }
+    return EMPM_OK;
+}
+
 static int check_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off, int ny,
                          int max_ny, int n_pairs, const float* sum_xy, const float* sum_yx, const int* nn_x,
                          const int* nn_y) {
@@ -170,7 +197,7 @@ extern "C" int empm_chamfer_workspace(int nx, int max_nx, int ny, int max_ny, in
     *bytes = 0;
     if ((double)n_pairs * max_nx * max_ny < 7e7 || (long long)nx + ny > (1LL << 30)) return EMPM_OK;
     const PointSets P{nullptr, nullptr, n_pairs, nx, nullptr, nullptr, n_pairs, ny};
-    *bytes = cellgrid_layout(P, 0, nullptr, nullptr);
+    *bytes = cellgrid_layout(P, 0, 2.f, nullptr, nullptr);
     return EMPM_OK;
 }
 
@@ -191,11 +218,12 @@ extern "C" int empm_chamfer_cells(const float* x, const int* x_off, int nx, int 
     CKL(cudaMemsetAsync(sum_yx, 0, sizeof(float) * n_pairs, s), "chamfer");
     const PointSets P{x, x_off, n_pairs, nx, y, y_off, n_pairs, ny};
     CellGridWork w;
-    cellgrid_layout(P, 0, workspace, &w);
-    CKL(cellgrid_build(P, 0, 2.f, w, s), "chamfer cell grids");
+    cellgrid_layout(P, 0, 2.f, workspace, &w);
+    CKL(cellgrid_build(P, 0, w, s), "chamfer cell grids");
     k_nn_cells<<<blocks_for((long long)nx + ny, kThreads), kThreads, 0, s>>>(P, w, nn_x, nn_y, sum_xy, sum_yx);
     CKL(cudaGetLastError(), "k_nn_cells");
-    return EMPM_OK;
+    return launch_nn(x, x_off, max_nx, y, y_off, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y, w.rest, w.rest_row,
+                     w.rest_row + nx, s);
 }
 
 extern "C" int empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,
@@ -206,15 +234,7 @@ extern "C" int empm_chamfer(const float* x, const int* x_off, int nx, int max_nx
     cudaStream_t s = (cudaStream_t)stream;
     CKL(cudaMemsetAsync(sum_xy, 0, sizeof(float) * n_pairs, s), "chamfer");
     CKL(cudaMemsetAsync(sum_yx, 0, sizeof(float) * n_pairs, s), "chamfer");
-    if (max_nx > 0) {
-        k_nn<<<dim3(blocks_for(max_nx, kThreads), n_pairs), kThreads, 0, s>>>(x, x_off, y, y_off, nn_x, sum_xy);
-        CKL(cudaGetLastError(), "k_nn (x -> y)");
-    }
-    if (max_ny > 0) {
-        k_nn<<<dim3(blocks_for(max_ny, kThreads), n_pairs), kThreads, 0, s>>>(y, y_off, x, x_off, nn_y, sum_yx);
-        CKL(cudaGetLastError(), "k_nn (y -> x)");
-    }
-    return EMPM_OK;
+    return launch_nn(x, x_off, max_nx, y, y_off, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y, nullptr, nullptr, nullptr, s);
 }
 
 extern "C" int empm_chamfer_backward(const float* x, const int* x_off, int nx, const float* y, const int* y_off,
