@@ -303,6 +303,7 @@ static __global__ void __launch_bounds__(256) k_bin_scatter(const PointSets P, i
 struct CellGridWork {
     SetGrid*  grids;
     unsigned* box;
+    double*   acc;      // one per set, zero after the build
     int*      start;    // bins + 1
     int*      sums;
     float4*   sorted;
@@ -325,7 +326,8 @@ inline size_t cellgrid_layout(const PointSets& P, int share, float per_cell, voi
     CellGridWork c;
     c.grids = (SetGrid*)take(sizeof(SetGrid) * P.sets());
     c.box = (unsigned*)take(sizeof(unsigned) * 6 * P.sets());
-    c.start = (int*)take(sizeof(int) * (bins + 1 + P.sets()));
+    c.acc = (double*)take(sizeof(double) * P.sets() + sizeof(int) * (bins + 1 + P.sets()));
+    c.start = base ? (int*)(c.acc + P.sets()) : nullptr;
     c.rest = base ? c.start + bins + 1 : nullptr;
     c.rest_row = (int*)take(sizeof(int) * (size_t)P.rows());
     c.sums = (int*)take(sizeof(int) * (bins / kScanTile + 1));
@@ -341,7 +343,7 @@ inline cudaError_t cellgrid_build(const PointSets& P, int share, const CellGridW
                                   cudaStream_t s) {
     const int n = P.rows(), sets = P.sets();
     const auto blocks = [](long long k, int t) { return (unsigned)((k + t - 1) / t); };
-    cudaError_t e = cudaMemsetAsync(w.start, 0, sizeof(int) * ((size_t)w.bins + 1 + sets), s);
+    cudaError_t e = cudaMemsetAsync(w.acc, 0, sizeof(double) * sets + sizeof(int) * ((size_t)w.bins + 1 + sets), s);
     if (e != cudaSuccess) return e;
     k_box_init<<<blocks(6LL * sets, 256), 256, 0, s>>>(w.box, 6 * sets);
     k_box<<<blocks(n, 256 * 16), 256, 0, s>>>(P, n, w.box);

@@ -28,9 +28,10 @@ inline int blocks_for(long long n, int threads) { return (int)((n + threads - 1)
 // For every query point q of pair blockIdx.y: nearest point of the pair's
 // target set, its squared distance added to sum[pair]. rest: only the pair's first
 // rest[pair] of the queries rest_row.
+template <typename Sum>
 __global__ void __launch_bounds__(kThreads) k_nn(const float* __restrict__ q, const int* __restrict__ q_off,
                                                  const float* __restrict__ t, const int* __restrict__ t_off,
-                                                 int* __restrict__ nn, float* __restrict__ sum,
+                                                 int* __restrict__ nn, Sum* __restrict__ sum,
                                                  const int* __restrict__ rest, const int* __restrict__ rest_row) {
     __shared__ float4 tile[kThreads];
     const int pair = blockIdx.y;
@@ -60,22 +61,23 @@ __global__ void __launch_bounds__(kThreads) k_nn(const float* __restrict__ q, co
     if (live) nn[i] = arg;
     // warp-level partial sums (every lane of the CTA is still here; lanes
     // without a query add zero), one atomic per warp
-    float v = (live && arg >= 0) ? best : 0.f;
+    Sum v = (live && arg >= 0) ? best : 0.f;
     for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-    if ((threadIdx.x & 31) == 0 && v != 0.f) atomicAdd(sum + pair, v);
+    if ((threadIdx.x & 31) == 0 && v != 0) atomicAdd(sum + pair, v);
 }
 
 // The same through cell grids: one thread per point of either cloud, in the order
 // of its own cloud's cells, searching the other cloud of its pair. Clouds of the
-// same size apart, the 27 cells around a query hold about 54 candidates.
+// same size apart, the 27 cells around a query hold about 54 candidates. The sums are
+// kept in 64 bits: in 32 their error was that of the order of the atomics, 1e-7 to
+// 5e-7 from run to run for 100,000 points.
 __global__ void __launch_bounds__(kThreads) k_nn_cells(const PointSets P, const CellGridWork w,
-                                                       int* __restrict__ nn_x, int* __restrict__ nn_y,
-                                                       float* __restrict__ sum_xy, float* __restrict__ sum_yx) {
-    __shared__ float part[kThreads / 32];
+                                                       int* __restrict__ nn_x, int* __restrict__ nn_y) {
+    __shared__ double part[kThreads / 32];
     __shared__ int ends[2];
     const int t = blockIdx.x * kThreads + threadIdx.x;
     const int n = P.rows();
-    float v = 0.f;
+    double v = 0.;
     int set = -1;
     if (t < n) {
         const bool in_a = t < P.rows_a;
@@ -94,24 +96,36 @@ __global__ void __launch_bounds__(kThreads) k_nn_cells(const PointSets P, const 
             w.rest_row[first + atomicAdd(w.rest + set, 1)] = __float_as_int(q.w);
         }
     }
-    // one atomic per block, or per thread where two clouds meet in it
+    // one atomic per block; where clouds meet in it per warp, or per thread
     if (threadIdx.x == 0) ends[0] = set;
     if (threadIdx.x == min(kThreads, n - (int)(blockIdx.x * kThreads)) - 1) ends[1] = set;
     __syncthreads();
-    float* sum = set < 0 ? nullptr : (set < P.sets_a ? sum_xy + set : sum_yx + (set - P.sets_a));
-    if (ends[0] != ends[1]) {
-        if (v != 0.f) atomicAdd(sum, v);
+    const bool one = ends[0] == ends[1];
+    if (!one && !__all_sync(0xffffffffu, set == __shfl_sync(0xffffffffu, set, 0) || set < 0)) {
+        if (v != 0.) atomicAdd(w.acc + set, v);
         return;
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+    if (!one) {
+        if ((threadIdx.x & 31) == 0 && v != 0.) atomicAdd(w.acc + set, v);
+        return;
+    }
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float s = 0.f;
+        double s = 0.;
         for (int k = 0; k < kThreads / 32; ++k) s += part[k];
-        if (s != 0.f) atomicAdd(sum, s);
+        if (s != 0.) atomicAdd(w.acc + set, s);
     }
+}
+
+__global__ void k_sums(const double* __restrict__ acc, int n_pairs, float* __restrict__ sum_xy,
+                       float* __restrict__ sum_yx) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n_pairs) return;
+    sum_xy[p] = (float)acc[p];
+    sum_yx[p] = (float)acc[n_pairs + p];
 }
 
 // Gradient in X of  g_xy[p] * sum_i |x_i - y_nn(i)|^2 + g_yx[p] * sum_j |y_j - x_nn(j)|^2
@@ -162,8 +176,9 @@ __global__ void k_pair_index(const int* off, int n_pairs, int* pair_of, int n) {
 
 // The brute-force search both ways. rest: only the queries left over by the cells
 // (counts of the x clouds, then of the y clouds).
+template <typename Sum>
 static int launch_nn(const float* x, const int* x_off, int max_nx, const float* y, const int* y_off, int max_ny,
-                     int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y, const int* rest,
+                     int n_pairs, Sum* sum_xy, Sum* sum_yx, int* nn_x, int* nn_y, const int* rest,
                      const int* rest_x, const int* rest_y, cudaStream_t s) {
     if (max_nx > 0) {
         k_nn<<<dim3(blocks_for(max_nx, kThreads), n_pairs), kThreads, 0, s>>>(x, x_off, y, y_off, nn_x, sum_xy, rest,
@@ -214,16 +229,18 @@ extern "C" int empm_chamfer_cells(const float* x, const int* x_off, int nx, int 
         return empm_set_error(nullptr, EMPM_ERR_INVALID, "chamfer: workspace of %zu bytes, 256-byte aligned, needed",
                               need);
     cudaStream_t s = (cudaStream_t)stream;
-    CKL(cudaMemsetAsync(sum_xy, 0, sizeof(float) * n_pairs, s), "chamfer");
-    CKL(cudaMemsetAsync(sum_yx, 0, sizeof(float) * n_pairs, s), "chamfer");
     const PointSets P{x, x_off, n_pairs, nx, y, y_off, n_pairs, ny};
     CellGridWork w;
     cellgrid_layout(P, 0, 2.f, workspace, &w);
     CKL(cellgrid_build(P, 0, w, s), "chamfer cell grids");
-    k_nn_cells<<<blocks_for((long long)nx + ny, kThreads), kThreads, 0, s>>>(P, w, nn_x, nn_y, sum_xy, sum_yx);
+    k_nn_cells<<<blocks_for((long long)nx + ny, kThreads), kThreads, 0, s>>>(P, w, nn_x, nn_y);
     CKL(cudaGetLastError(), "k_nn_cells");
-    return launch_nn(x, x_off, max_nx, y, y_off, max_ny, n_pairs, sum_xy, sum_yx, nn_x, nn_y, w.rest, w.rest_row,
-                     w.rest_row + nx, s);
+    const int rn = launch_nn(x, x_off, max_nx, y, y_off, max_ny, n_pairs, w.acc, w.acc + n_pairs, nn_x, nn_y, w.rest,
+                             w.rest_row, w.rest_row + nx, s);
+    if (rn) return rn;
+    k_sums<<<blocks_for(n_pairs, 256), 256, 0, s>>>(w.acc, n_pairs, sum_xy, sum_yx);
+    CKL(cudaGetLastError(), "k_sums");
+    return EMPM_OK;
 }
 
 extern "C" int empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,

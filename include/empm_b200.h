@@ -537,8 +537,8 @@ int  empm_chamfer(const float* x, const int* x_off, int nx, int max_nx, const fl
 
 /* The same through cell grids of the clouds, in a caller's device workspace of
  * empm_chamfer_workspace bytes (256-byte aligned; 0 bytes: the clouds are small and
- * searched by brute force). Neighbours are the same; the sums differ by the order
- * of their single-precision additions. */
+ * searched by brute force). Neighbours are the same; the sums are
+ * added in 64 bits and rounded once. */
 int  empm_chamfer_workspace(int nx, int max_nx, int ny, int max_ny, int n_pairs, size_t* bytes);
 int  empm_chamfer_cells(const float* x, const int* x_off, int nx, int max_nx, const float* y, const int* y_off,
                         int ny, int max_ny, int n_pairs, float* sum_xy, float* sum_yx, int* nn_x, int* nn_y,
