@@ -300,9 +300,9 @@ void constitutive_call(ConstitutiveCall* io, float dt, const MaterialScalars* ms
     io->changed = o.mat_changed;
 }
 
-// The update of rollouts. The kernels of a tape, and of rollouts whose states a tape
-// starts from, take constitutive_general: their
-// adjoint differentiates the decomposition, whose singular values enter the
+// The update of rollouts in cell order. Single substeps, whatever their size and route,
+// the kernels of a tape, and rollouts whose states a tape starts from take
+// constitutive_general: the adjoint differentiates the decomposition, whose singular values enter the
 // gradients in E and nu with a bias of 1e-7 of a strain of 1e-4; the same one in the
 // forward pass belongs to the values that callers have compared with so far (the
 // branch without it moves those gradients by 5e-4 to 9e-4 of themselves, four to

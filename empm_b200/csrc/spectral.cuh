@@ -8,7 +8,7 @@
 //   tau       = U diag(h(s)) U^T   (symmetric, so its symmetrisation is exact),
 // where f and h also depend on mu, lam and the yield stress, and the return
 // map updates those three. `spectral_map` evaluates f, h and the updated
-// scalars. It mirrors constitutive() in constitutive.cuh operation for
+// scalars. It mirrors constitutive_general() in constitutive.cuh operation for
 // operation, so it takes the same branches. Evaluated on Dual<6> numbers
 // seeded on (s0, s1, s2, mu, lam, yield), it yields the Jacobian that the
 // adjoint needs.
@@ -228,7 +228,7 @@ EMPM_HD void spectral_fcr_elastic(const float s[3], float mu, float lam, float y
     o.ys = dseed<6>(ys, 5);
 }
 
-// The von Mises yield test of constitutive() (constitutive.cuh) on the
+// The von Mises yield test of constitutive_general() (constitutive.cuh) on the
 // singular values: true when the return map changes nothing.
 EMPM_HD bool von_mises_inside(const float s[3], float mu, float lam, float ys, bool damage) {
     const V3 sig = v3(fmaxf(s[0], 0.01f), fmaxf(s[1], 0.01f), fmaxf(s[2], 0.01f));

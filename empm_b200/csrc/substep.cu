@@ -682,8 +682,8 @@ static int launch_p2g_single(EmpmCtx* ctx, const ParticleArrays& P, const Materi
     CK(cudaGetLastError(), "k_order_ranges");
     k_order_fill<<<blocks_for(n, 256), 256, 0, stream>>>(ob.keys, ob.offsets, ob.order, n);
     CK(cudaGetLastError(), "k_order_fill");
-    launch_p2g_cells<false>(few_particles(ctx, n), stream, P, M, Fe, L, ctx->grid_mom, ctx->flags,
-                            uniform_material(ctx), ob.order);
+    launch_p2g_cells<true>(few_particles(ctx, n), stream, P, M, Fe, L, ctx->grid_mom, ctx->flags,
+                           uniform_material(ctx), ob.order);
     CK(cudaGetLastError(), "k_p2g_cells (ordered)");
     return EMPM_OK;
 }
