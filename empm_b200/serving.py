@@ -547,9 +547,10 @@ class GpuExecutor:
         mat = N.EmpmMaterial(self.mat["vol"][self.ai].data_ptr(), self.mat["mu"][self.ai].data_ptr(),
                              self.mat["lam"][self.ai].data_ptr(), self.mat["ys"][self.ai].data_ptr(), None,
                              self.Fe.data_ptr())
-        # the block's boundaries are checkpoints of the gradient requests among them
-        flags = N.ROLLOUT_TAPE if any(t.req.grad for t in active) else 0
-        N.check(self.L.empm_rollout_ex(self.ctx, views[0], views[1], mat, table, n_tables, L, flags,
+        # the block's boundaries are the checkpoints of its gradient requests; every block
+        # takes the tape's update, so that a plain request's result does not depend on
+        # the requests beside it
+        N.check(self.L.empm_rollout_ex(self.ctx, views[0], views[1], mat, table, n_tables, L, N.ROLLOUT_TAPE,
                                        self._sptr(self.fwd_stream)), self.ctx)
         if L % 2 == 1:
             self.cur = 1 - c
