@@ -77,10 +77,10 @@ struct SortedBuffers {
     size_t scan_tmp_bytes = 0;
 };
 
-// Buffers that order the particles of a single substep by cell: one block, allocated
-// on first use.
+// Buffers that order the particles of a single substep by cell: a part of the grid's
+// block in contexts of one instance, else a block of their own, allocated on first use.
 struct OrderBuffers {
-    bool      allocated = false;
+    char*     own = nullptr;               // block of their own
     int       n = 0;                       // particle capacity
     long long nb = 0;                      // block capacity
     int2*     keys = nullptr;              // [n] cell and rank in it
@@ -137,6 +137,7 @@ struct EmpmCtx {
     int          device = 0;
     int          sm_count = 148;
     size_t       step_entries = 0;         // capacity of the step-table array, in EmpmStep entries
+    char*        grid_block = nullptr;     // the buffers of the grid, one allocation
     float4*      grid_mom = nullptr;       // P2G accumulation (px, py, pz, m), blocked layout; zero between substeps
     float4*      grid_vel = nullptr;       // node velocity after the grid update, blocked layout
     unsigned char* flags = nullptr;        // touched node blocks of the current substep

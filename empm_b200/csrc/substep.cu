@@ -127,9 +127,77 @@ static void free_sorted(SortedBuffers& sb) {
     sb = SortedBuffers();
 }
 
+// From this many particles on a single substep's P2G goes over the particles in cell
+// order (k_order_*, then the per-cell scatter with the state read through the order)
+// instead of in the caller's (k_p2g_direct, bound by its 27 reductions per particle).
+// Particles in random order, the P2G with its ordering, us:
+//   n       16k    30k    60k   120k   250k   500k    1M
+//   direct  17.4   25.3   39.5   80.3  163.6  284.5  462.2
+//   order   15.6   15.5   23.2   33.1   60.2  106.3  214.7
+// Below the line the calls wait on the host (90 us each from Python) and three more
+// launches would cost it 7 us. More than 64 cells per particle keep the direct kernel:
+// the counts would outgrow the particles' state. The G2P stays in the caller's order
+// (500k: 57.8 us; through the order 81, its scattered stores).
+constexpr int kOrderMin = 65536;
+
+static size_t pad256(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+
+// Bytes of the order's buffers, of which the first *zero are to be zero.
+static size_t order_bytes(int n, long long nb, size_t* zero) {
+    *zero = pad256(sizeof(int) * 64 * (size_t)nb + (size_t)nb);
+    return *zero + sizeof(int) * 64 * (size_t)nb + pad256(sizeof(int) * (size_t)n) + sizeof(int2) * (size_t)n +
+           sizeof(int);
+}
+
+static void order_place(OrderBuffers& ob, char* base, int n, long long nb) {
+    size_t zero = 0;
+    order_bytes(n, nb, &zero);
+    ob.n = n;
+    ob.nb = nb;
+    ob.counts = reinterpret_cast<int*>(base);
+    ob.marks = reinterpret_cast<unsigned char*>(ob.counts + 64 * nb);
+    ob.offsets = reinterpret_cast<int*>(base + zero);
+    ob.order = ob.offsets + 64 * nb;
+    ob.keys = reinterpret_cast<int2*>(reinterpret_cast<char*>(ob.order) + pad256(sizeof(int) * (size_t)n));
+    ob.next = reinterpret_cast<int*>(ob.keys + n);
+}
+
 static void free_order(OrderBuffers& ob) {
-    if (ob.keys) cudaFree(ob.keys);   // the others are parts of its block
+    if (ob.own) cudaFree(ob.own);
     ob = OrderBuffers();
+}
+
+// The grid's buffers at the context's capacity, in one allocation, cleared; with those
+// of the order where the context's single substeps will take it (one instance, the line
+// above) and there is room. An allocation takes the driver 0.35 ms whatever its size (0.3
+// to give back), more than the order gains the substep that makes it: 500k particles, a
+// new context's first substep 0.57 ms with the buffers allocated in it, 0.22 now, 0.37 by
+// the direct kernel; creation 1.1 ms, 1.4 with an allocation per buffer.
+static cudaError_t alloc_grid(EmpmCtx* ctx, bool with_order) {
+    if (ctx->grid_block) cudaFree(ctx->grid_block);
+    free_order(ctx->ob);
+    ctx->grid_block = nullptr;
+    ctx->grid_mom = ctx->grid_vel = nullptr;
+    ctx->flags = nullptr;
+    const size_t cb = (size_t)ctx->cap_blocks, nodes = cb * 64 * sizeof(float4), grid = 2 * nodes + pad256(cb);
+    with_order = with_order && ctx->cap_particles >= kOrderMin && ctx->cap_blocks <= ctx->cap_particles;
+    size_t zero = 0;
+    const size_t order = with_order ? order_bytes(ctx->cap_particles, ctx->cap_blocks, &zero) : 0;
+    char* base = nullptr;
+    cudaError_t e = cudaMalloc(&base, grid + order);
+    if (e != cudaSuccess && with_order) {
+        cudaGetLastError();
+        with_order = false;
+        zero = 0;
+        e = cudaMalloc(&base, grid);
+    }
+    if (e != cudaSuccess) return e;
+    ctx->grid_block = base;
+    ctx->grid_mom = reinterpret_cast<float4*>(base);
+    ctx->grid_vel = reinterpret_cast<float4*>(base + nodes);
+    ctx->flags = reinterpret_cast<unsigned char*>(base + 2 * nodes);
+    if (with_order) order_place(ctx->ob, base + grid, ctx->cap_particles, ctx->cap_blocks);
+    return cudaMemset(base, 0, grid + zero);
 }
 
 static void free_store(AdjointBuffers& ab) {
@@ -248,17 +316,11 @@ extern "C" int empm_batch_create(const EmpmModelParams* params, const int* n_par
     ctx->cap_particles = (int)total;
     ctx->cap_blocks = blocks;
     ctx->cap_inst = n_instances;
-    const size_t grid_bytes = (size_t)blocks * 64 * sizeof(float4);
     cudaError_t e = cudaGetDevice(&ctx->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_inst, sizeof(InstanceConsts) * n_instances);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->grid_mom, grid_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->grid_vel, grid_bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->flags, (size_t)blocks);
+    if (e == cudaSuccess) e = alloc_grid(ctx, n_instances == 1);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(ctx->grid_mom, 0, grid_bytes);
-    if (e == cudaSuccess) e = cudaMemset(ctx->grid_vel, 0, grid_bytes);
-    if (e == cudaSuccess) e = cudaMemset(ctx->flags, 0, (size_t)blocks);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_a, cudaEventDisableTiming);
@@ -289,7 +351,7 @@ extern "C" int empm_ctx_destroy(EmpmCtx* ctx) {
     free_sorted(ctx->sb);
     free_order(ctx->ob);
     free_adjoint(ctx->adj);
-    void* ptrs[] = {ctx->d_inst, ctx->grid_mom, ctx->grid_vel, ctx->flags, ctx->d_steps, ctx->d_status};
+    void* ptrs[] = {ctx->d_inst, ctx->grid_block, ctx->d_steps, ctx->d_status};
     for (void* q : ptrs) if (q) cudaFree(q);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->ev_a) cudaEventDestroy(ctx->ev_a);
@@ -357,19 +419,8 @@ extern "C" int empm_batch_reserve(EmpmCtx* ctx, int max_particles, long long max
     destroy_graphs(ctx);
     ctx->resident = false;
     if (grow_b) {
-        const size_t grid_bytes = (size_t)max_blocks * 64 * sizeof(float4);
-        cudaFree(ctx->grid_mom);
-        cudaFree(ctx->grid_vel);
-        cudaFree(ctx->flags);
-        ctx->grid_mom = ctx->grid_vel = nullptr;
-        ctx->flags = nullptr;
-        CK(cudaMalloc(&ctx->grid_mom, grid_bytes), "reserve grid");
-        CK(cudaMalloc(&ctx->grid_vel, grid_bytes), "reserve grid");
-        CK(cudaMalloc(&ctx->flags, (size_t)max_blocks), "reserve grid");
-        CK(cudaMemset(ctx->grid_mom, 0, grid_bytes), "reserve grid");
-        CK(cudaMemset(ctx->grid_vel, 0, grid_bytes), "reserve grid");
-        CK(cudaMemset(ctx->flags, 0, (size_t)max_blocks), "reserve grid");
         ctx->cap_blocks = max_blocks;
+        CK(alloc_grid(ctx, false), "reserve grid");
     }
     if (grow_i) {
         cudaFree(ctx->d_inst);
@@ -381,7 +432,7 @@ extern "C" int empm_batch_reserve(EmpmCtx* ctx, int max_particles, long long max
     }
     if (grow_p) ctx->cap_particles = max_particles;
     free_sorted(ctx->sb);       // re-allocated at the new capacity on next use
-    free_order(ctx->ob);
+    if (ctx->ob.n < ctx->cap_particles) free_order(ctx->ob);
     free_adjoint(ctx->adj);
     // step tables for blocks of up to 128 substeps of max_instances instances
     const size_t entries = (size_t)128 * ctx->cap_inst;
@@ -615,52 +666,30 @@ static int launch_grid_update(EmpmCtx* ctx, int table, cudaStream_t stream) {
     return rc;
 }
 
-// From this many particles on a single substep's P2G goes over the particles in cell
-// order (k_order_*, then the per-cell scatter with the state read through the order)
-// instead of in the caller's (k_p2g_direct, bound by its 27 reductions per particle).
-// Particles in random order, the P2G with its ordering, us:
-//   n       16k    30k    60k   120k   250k   500k    1M
-//   direct  17.4   25.3   39.5   80.3  163.6  284.5  462.2
-//   order   15.6   15.5   23.2   33.1   60.2  106.3  214.7
-// Below the line the calls wait on the host (90 us each from Python) and three more
-// launches would cost it 7 us. More than 64 cells per particle keep the direct kernel:
-// the counts would outgrow the particles' state. The G2P stays in the caller's order
-// (500k: 57.8 us; through the order 81, its scattered stores).
-constexpr int kOrderMin = 65536;
-
 static bool use_order(EmpmCtx* ctx, cudaStream_t stream) {
     const long long n = ctx->n_particles;
     if (ctx->sort_every <= 0 || ctx->p2g_mode != 2 || n < kOrderMin || ctx->nblocks > n) return false;
     OrderBuffers& ob = ctx->ob;
-    if (ob.allocated && ob.n >= n && ob.nb >= ctx->nblocks) return true;
-    // nothing is allocated while the caller captures, and without room for the
-    // buffers the direct kernel needs none
+    if (ob.keys && ob.n >= n && ob.nb >= ctx->nblocks) return true;
+    // a batch, or a context made larger: nothing is allocated while the caller
+    // captures, and without room for the buffers the direct kernel needs none
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return false;
     }
     free_order(ob);
-    const size_t cn = ((size_t)ctx->cap_particles + 3) & ~(size_t)3, cb = (size_t)ctx->cap_blocks;
-    // one block: keys, order, counts and marks (zero from here on), offsets, next
-    const size_t zero = sizeof(int) * 64 * cb + cb, bytes = sizeof(int) * (3 * cn + 64 * cb + 1) + ((zero + 15) & ~(size_t)15);
-    char* base = nullptr;
-    cudaError_t e = cudaMalloc(&base, bytes);
-    ob.keys = reinterpret_cast<int2*>(base);
-    if (e == cudaSuccess) e = cudaMemsetAsync(base + sizeof(int) * 3 * cn, 0, zero, stream);
+    const long long nb = std::min(ctx->cap_blocks, (long long)ctx->cap_particles);
+    size_t zero = 0;
+    const size_t bytes = order_bytes(ctx->cap_particles, nb, &zero);
+    cudaError_t e = cudaMalloc(&ob.own, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ob.own, 0, zero, stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         free_order(ob);
         return false;
     }
-    ob.order = reinterpret_cast<int*>(base + sizeof(int) * 2 * cn);
-    ob.counts = ob.order + cn;
-    ob.marks = reinterpret_cast<unsigned char*>(ob.counts + 64 * cb);
-    ob.offsets = reinterpret_cast<int*>(base + sizeof(int) * 3 * cn + ((zero + 15) & ~(size_t)15));
-    ob.next = ob.offsets + 64 * cb;
-    ob.allocated = true;
-    ob.n = (int)cn;
-    ob.nb = (long long)cb;
+    order_place(ob, ob.own, ctx->cap_particles, nb);
     return true;
 }
 

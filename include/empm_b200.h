@@ -267,10 +267,11 @@ int  empm_unpack_particles(const EmpmParticles* src, float* x3, float* v3, float
 
 /* One MLS-MPM substep: in -> out (distinct buffers). step is a host array of
  * one schedule per instance (n_instances entries), copied to the device on
- * the given stream. From 65,536 particles on a context allocates 12 bytes per
- * particle and 8 per grid cell at its first substep (here and in place), to put the
- * particles of a cell next to one another; where there is no room, or the stream
- * is being captured, the substep runs without. */
+ * the given stream. From 65,536 particles on, with no more grid blocks than particles, a
+ * context holds 12 bytes per particle and 8 per grid cell besides its grid, to put the
+ * particles of a cell next to one another: from its creation with one instance, from its
+ * first such substep (here or in place) with several or after empm_batch_reserve. Where
+ * there is no room, or that substep is being captured, it runs without. */
 int  empm_substep(EmpmCtx* ctx, const EmpmParticles* in, EmpmParticles* out,
                   const EmpmMaterial* mat, const EmpmStep* step, void* stream);
 
