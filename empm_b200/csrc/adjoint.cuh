@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(NT, MINB) k_adj_g2p(const AdjG2PArgs a) {
     if (valid)
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
-            b[e] = base_node(xs[e], c.inv_dx);
+            b[e] = base_unclamped(xs[e], c.inv_dx);
             fx[e] = base_frac(xs[e], c.inv_dx, b[e]);
         }
     const CellSlot cell = cell_scatter_slot(sh, valid, b, c.G, c.NB, c.boff);

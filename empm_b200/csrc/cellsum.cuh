@@ -54,7 +54,7 @@ struct CellSlot {
 };
 
 // Groups of equal cells over the warp; every thread of the CTA takes part.
-// valid: the thread has a particle, with base node b in an instance's grid of
+// valid: the thread has a particle, with base node b (unclamped) in an instance's grid of
 // resolution G.
 template <bool MASS, int NT>
 __device__ __forceinline__ CellSlot cell_scatter_slot(CellScatter<MASS, NT>& sh, bool valid, const int b[3], int G,
@@ -65,7 +65,7 @@ __device__ __forceinline__ CellSlot cell_scatter_slot(CellScatter<MASS, NT>& sh,
     c.NB = NB;
     c.base = -1;
     unsigned key = 0xffffffffu;
-    if (valid && b[0] >= 0 && b[1] >= 0 && b[2] >= 0 && b[0] + 2 < G && b[1] + 2 < G && b[2] + 2 < G) {
+    if (valid && axis_in_grid(b[0], G) && axis_in_grid(b[1], G) && axis_in_grid(b[2], G)) {
         key = ((unsigned)(boff + block_of(b[0], b[1], b[2], NB)) << 6) | ((b[0] & 3) << 4) | ((b[1] & 3) << 2) |
               (b[2] & 3);
         c.base = (b[0] << 20) | (b[1] << 10) | b[2];
@@ -174,7 +174,7 @@ __device__ __noinline__ void cell_scatter_edge(const CellScatter<MASS, NT>* sh, 
     const CellTerms c = cell_scatter_get(*sh, slot);
     for (int n = 0; n < 27; ++n) {
         const int i = n / 9, j = (n / 3) % 3, k = n % 3;
-        const int ix = bx + i, iy = by + j, iz = bz + k;
+        const int ix = base_clamp(bx) + i, iy = base_clamp(by) + j, iz = base_clamp(bz) + k;
         if (ix < 0 || iy < 0 || iz < 0 || ix >= G || iy >= G || iz >= G) continue;
         float wx, wy, ux, uy;
         bspline_at(c.fx, i, wx, ux);

@@ -146,8 +146,7 @@ EMPM_HD StencilAddr stencil_addr(int boff, int NB, const int b[3]) {
 
 // stencil node (i, j, k) inside the instance's grid (for stencils that are not entirely inside)
 EMPM_HD bool node_in_grid(const int b[3], int i, int j, int k, int G) {
-    const int ix = b[0] + i, iy = b[1] + j, iz = b[2] + k;
-    return ix >= 0 && iy >= 0 && iz >= 0 && ix < G && iy < G && iz < G;
+    return (unsigned)b[0] + i < (unsigned)G && (unsigned)b[1] + j < (unsigned)G && (unsigned)b[2] + k < (unsigned)G;
 }
 
 // -------------------------------------------------------------------------
@@ -200,7 +199,7 @@ __device__ __forceinline__ bool prepare_particle(const ParticleArrays& P, const 
 __device__ __forceinline__ void mark_stencil_blocks(unsigned char* flags, const Stencil& st, const StepConsts& c) {
     const int G = c.G;
     const int lo[3] = {max(st.b[0], 0), max(st.b[1], 0), max(st.b[2], 0)};
-    const int hi[3] = {min(st.b[0] + 2, G - 1), min(st.b[1] + 2, G - 1), min(st.b[2] + 2, G - 1)};
+    const int hi[3] = {min(st.b[0], G - 3) + 2, min(st.b[1], G - 3) + 2, min(st.b[2], G - 3) + 2};
     for (int bi = lo[0] >> 2; bi <= hi[0] >> 2; ++bi)
         for (int bj = lo[1] >> 2; bj <= hi[1] >> 2; ++bj)
             for (int bk = lo[2] >> 2; bk <= hi[2] >> 2; ++bk) flags[c.boff + (bi * c.NB + bj) * c.NB + bk] = 1;
@@ -533,9 +532,9 @@ __device__ __forceinline__ G2POut g2p_move(CellScatter<true, NT>& sh, const Step
     bool in_grid = true;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        b[a] = base_node(xs[a], c.inv_dx);
+        b[a] = base_unclamped(xs[a], c.inv_dx);
         fx[a] = base_frac(xs[a], c.inv_dx, b[a]);
-        in_grid = in_grid && b[a] >= 0 && b[a] + 2 < c.G;
+        in_grid = in_grid && axis_in_grid(b[a], c.G);
     }
     G2POut o;
     if (in_grid) {
@@ -761,7 +760,7 @@ __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid,
     int b[3] = {0, 0, 0};
     if (valid)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) b[a] = base_node(xs[a], c.inv_dx);
+        for (int a = 0; a < 3; ++a) b[a] = base_unclamped(xs[a], c.inv_dx);
     const CellSlot cell = cell_scatter_slot(sh, valid, b, c.G, c.NB, c.boff);
     if (valid) {
         if (sp.n_modifiers > 0) {
@@ -1068,7 +1067,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_p2g_tiled(const TiledArgs a
                     // same cell do not hit the same shared-memory node together
                     int s = (int)(threadIdx.x % 27u);
                     int i = s / 9, j = (s / 3) % 3, k = s % 3;
-                    const int li0 = q.st.b[0] - tb.o[0], lj0 = q.st.b[1] - tb.o[1], lk0 = q.st.b[2] - tb.o[2];
+                    const int li0 = base_clamp(q.st.b[0]) - tb.o[0], lj0 = base_clamp(q.st.b[1]) - tb.o[1],
+                              lk0 = base_clamp(q.st.b[2]) - tb.o[2];
                     for (int it = 0; it < 27; ++it) {
                         const float4 v = p2g_node_dyn(pre, i, j, k);
                         float* dst = reinterpret_cast<float*>(tile + ((li0 + i) * tb.e[1] + (lj0 + j)) * tb.e[2] + (lk0 + k));

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(128) k_restart_p2g(ParticleArrays P, const flo
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const int ix = st.b[0] + i, iy = st.b[1] + j, iz = st.b[2] + k;
-                if (!in_grid && (ix < 0 || iy < 0 || iz < 0 || ix >= c.G || iy >= c.G || iz >= c.G)) continue;
+                if (!in_grid && !node_in_grid(st.b, i, j, k, c.G)) continue;
                 const float wm = st.w[0][i] * st.w[1][j] * st.w[2][k] * xm.w;
                 red_add_v4(grid + gaddr(c, ix, iy, iz), make_float4(wm * disp.x, wm * disp.y, wm * disp.z, wm));
             }

@@ -26,18 +26,28 @@ struct Stencil {
 // subtraction fused into one rounding. Every kernel derives a particle's base
 // node from this function (stencils, cell keys, shared-memory tile boxes),
 // so they agree bit for bit whatever the compiler does with separate
-// multiply-adds.
-EMPM_HD int base_node(float x, float inv_dx) { return (int)fmaf(x, inv_dx, -0.5f); }
+// multiply-adds. The conversion saturates, so base + 2 overflows for a
+// particle 2^31 cells away: the tests of a stencil against the grid do without the
+// sum or add as unsigned, all else takes clamped bases.
+EMPM_HD int base_unclamped(float x, float inv_dx) { return (int)fmaf(x, inv_dx, -0.5f); }
+
+// Bases whose nodes are all outside any grid (of 1024 at most) are one of two: sums like
+// base + 2 and the volume of a tile's box then stay in an int.
+EMPM_HD int base_clamp(int b) { return b < -4 ? -4 : (b > 1028 ? 1028 : b); }
+EMPM_HD int base_node(float x, float inv_dx) { return base_clamp(base_unclamped(x, inv_dx)); }
+
+// 0 <= b and b + 2 < G for any b (G >= 4)
+EMPM_HD bool axis_in_grid(int b, int G) { return (unsigned)b < (unsigned)(G - 2); }
 
 // fx = x * inv_dx - base, rounded once.
-EMPM_HD float base_frac(float x, float inv_dx, int b) { return fmaf(x, inv_dx, -(float)b); }
+EMPM_HD float base_frac(float x, float inv_dx, int unclamped) { return fmaf(x, inv_dx, -(float)unclamped); }
 
 EMPM_HD Stencil make_stencil(V3 x, float inv_dx) {
     Stencil st;
     const float xs[3] = {x.x, x.y, x.z};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        st.b[a] = base_node(xs[a], inv_dx);
+        st.b[a] = base_unclamped(xs[a], inv_dx);
         const float f = base_frac(xs[a], inv_dx, st.b[a]);
         st.fx[a] = f;
         const float wa = 1.5f - f, wb = f - 1.f, wc = f - 0.5f;
@@ -67,8 +77,7 @@ EMPM_HD void bspline_at(float f, int i, float& w, float& dw) {
 }
 
 EMPM_HD bool stencil_in_grid(const Stencil& st, int G) {
-    return st.b[0] >= 0 && st.b[1] >= 0 && st.b[2] >= 0 &&
-           st.b[0] + 2 < G && st.b[1] + 2 < G && st.b[2] + 2 < G;
+    return axis_in_grid(st.b[0], G) && axis_in_grid(st.b[1], G) && axis_in_grid(st.b[2], G);
 }
 
 // Pre-P2G particle velocity modifiers (mpm_solver_diff.py:977-991, 1022-1036,
