@@ -20,6 +20,7 @@ from typing import Optional, Sequence, Union
 
 import torch
 from torch import Tensor
+from torch.utils._python_dispatch import is_in_torch_dispatch_mode
 
 from . import _native as N
 
@@ -47,7 +48,10 @@ def _f9_pack(dst: Tensor, m: Tensor) -> None:
 
 
 def _f9_unpack(src: Tensor, n: int) -> Tensor:
+    # the kernel where nothing records the call: a trace would keep its output's
+    # allocation and lose what fills it
     if n > 0 and type(src) is Tensor and src.is_cuda and src.dtype == DTYPE and not src.requires_grad \
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling() and not is_in_torch_dispatch_mode() \
             and src.is_contiguous() and src.numel() >= 9 * n and src.data_ptr() % 16 == 0:
         out = torch.empty((n, 3, 3), dtype=DTYPE, device=src.device)
         with torch.cuda.device(src.device):
