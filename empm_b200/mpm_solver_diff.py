@@ -332,7 +332,11 @@ class MPMWARPDiff(object):
         """(collider, modifier) windows for empm_schedule_fill, or None where the
         substeps need the general path: modify callbacks other than _move_point,
         layered releases (their threshold changes), one parameter block under two
-        registrations, and times whose arithmetic is not that of a double."""
+        registrations, times whose arithmetic is not that of a double, and solvers
+        that resolve their substeps in their own way."""
+        if any(getattr(getattr(self, k), "__func__", getattr(self, k)) is not getattr(f, "__func__", f)
+               for k, f in _RESOLVE.items()):
+            return None
         colliders, modify = self.collider_params, self.modify_bc
         mods = list(self.impulse_params) + list(self.particle_velocity_modifier_params)
         if type(t) is not float or type(dt) is not float or not math.isfinite(t) or not math.isfinite(dt) \
@@ -722,3 +726,7 @@ class MPMWARPDiff(object):
             cov = mpm_state.particle_cov.data_ptr() if getattr(mpm_model, "update_cov_with_F", False) else None
             N.check(ctx.L.empm_restart_F(ctx.ptr, mpm_state._particles(), tgt.data_ptr(), mpm_state._sel_ptr(), cov,
                                          _stream_ptr(mpm_state.device)), ctx.ptr)
+
+
+# what empm_schedule_fill does natively
+_RESOLVE = {k: getattr(MPMWARPDiff, k) for k in ("_fill_step", "_gate", "_window", "_modify", "_move_point")}
