@@ -8,7 +8,8 @@ substeps of the caller's own workload under each candidate:
 * ``sort_every``: the period of the cell sort (8, 16, 32 substeps);
 * ``p2g_mode`` / ``tile_cap`` / ``seg_cap``: contributions summed per cell, or
   accumulation in a per-CTA shared-memory node tile of 512 / 1024 / 2048 nodes
-  (the tile shape); ``seg_cap`` no longer changes a launch;
+  (the tile shape); candidates that differ in ``seg_cap`` alone launch the same
+  and are timed once;
 * ``g2p_tile``: G2P gathering directly from L2 or from a staged tile;
 * ``fuse``: the G2P of each substep and the stress + P2G of the next as one
   kernel between cell sorts, or separate kernels.
@@ -89,6 +90,14 @@ def _apply(target, opts: Dict[str, int]) -> None:
         setattr(target, k, bool(v) if k in ("g2p_tile", "fuse") else int(v))
 
 
+def _timed_once(cands: List[Dict[str, int]]) -> List[List[Dict[str, int]]]:
+    """The candidates in groups of equal launches, in their order."""
+    groups: Dict[tuple, List[Dict[str, int]]] = {}
+    for c in cands:
+        groups.setdefault(tuple(c.get(k, DEFAULTS[k]) for k in OPTION_NAMES if k != "seg_cap"), []).append(c)
+    return list(groups.values())
+
+
 def tune_batch(batch, dt: float, substeps: int = 32, candidates: Optional[List[Dict[str, int]]] = None,
                path: Optional[str] = None, force: bool = False) -> Dict:
     """Pick the fastest launch options for a BatchedMPM on its current state.
@@ -124,8 +133,8 @@ def tune_batch(batch, dt: float, substeps: int = 32, candidates: Optional[List[D
 
     times = {}
     batch.use_graph = True
-    for cand in cands:
-        _apply(batch, cand)
+    for group in _timed_once(cands):
+        _apply(batch, group[0])
         restore()
         batch.rollout(dt, substeps, block=substeps)        # captures this candidate's graph
         restore()
@@ -135,7 +144,7 @@ def tune_batch(batch, dt: float, substeps: int = 32, candidates: Optional[List[D
         batch.rollout(dt, substeps, block=substeps)
         e1.record()
         torch.cuda.synchronize()
-        times[json.dumps(cand, sort_keys=True)] = e0.elapsed_time(e1) / substeps
+        times.update((json.dumps(c, sort_keys=True), e0.elapsed_time(e1) / substeps) for c in group)
     restore()
     batch.use_graph = saved["use_graph"]
     best = json.loads(min(times, key=times.get))
@@ -178,8 +187,8 @@ def tune_solver(solver, model, state, dt: float, substeps: int = 32,
         solver.time = t0
 
     times = {}
-    for cand in cands:
-        _apply(solver, cand)
+    for group in _timed_once(cands):
+        _apply(solver, group[0])
         restore()
         solver.rollout(model, state, other, dt, substeps, schedule=schedule)
         restore()
@@ -189,7 +198,7 @@ def tune_solver(solver, model, state, dt: float, substeps: int = 32,
         solver.rollout(model, state, other, dt, substeps, schedule=schedule)
         e1.record()
         torch.cuda.synchronize()
-        times[json.dumps(cand, sort_keys=True)] = e0.elapsed_time(e1) / substeps
+        times.update((json.dumps(c, sort_keys=True), e0.elapsed_time(e1) / substeps) for c in group)
     restore()
     best = json.loads(min(times, key=times.get))
     _apply(solver, best)

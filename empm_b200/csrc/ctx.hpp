@@ -17,7 +17,6 @@ struct GraphKey {
     int           p2g_mode;
     int           g2p_tile;
     int           tile_cap;
-    int           seg_cap;
     int           fuse;                       // fused G2P + P2G runs in use (option and hold pattern)
     unsigned long long params_version;
     int           flags;                      // EMPM_ROLLOUT_RESUME / EMPM_ROLLOUT_KEEP
@@ -30,7 +29,7 @@ struct GraphKey {
 struct SegGraphKey {
     unsigned long long epoch;
     unsigned long long params_version;
-    int                seg_cap, p2g_mode, sort_every, n;
+    int                p2g_mode, sort_every, n;
     int                n_steps, store;
     const void*        buf[10];
 };
@@ -164,7 +163,6 @@ struct EmpmCtx {
     int          p2g_mode = 2;             // 0 direct reductions, 1 shared-memory tile, 2 summed per cell
     int          g2p_tile = 0;
     int          tile_cap = 1024;          // nodes per shared-memory tile (16 B each)
-    int          seg_cap = 4;              // accepted, without effect
     int          adj_store = 1;            // adjoint segments store substep grids instead of recomputing
     int          fuse = 1;                 // sorted rollouts fuse the G2P of one substep with the P2G of the next
     bool         fuse_ok = true;           // the uploaded step tables allow it (holds never released)

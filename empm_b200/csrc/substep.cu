@@ -385,8 +385,8 @@ extern "C" int empm_ctx_set_option(EmpmCtx* ctx, int option, int value) {
         case EMPM_OPT_SEG_CAP:
             if (value < 1 || value > 32 || (value & (value - 1)) != 0)
                 return empm_set_error(ctx, EMPM_ERR_INVALID, "seg_cap %d not a power of two in 1..32", value);
-            ctx->seg_cap = value;
-            break;
+            ctx->resident = false;
+            return EMPM_OK;   // without effect: launches and captured graphs stay as they are
         default: return empm_set_error(ctx, EMPM_ERR_INVALID, "unknown option %d", option);
     }
     invalidate_graphs(ctx);
@@ -1171,7 +1171,6 @@ extern "C" int empm_rollout_ex(EmpmCtx* ctx, EmpmParticles* a, EmpmParticles* b,
         key.p2g_mode = ctx->p2g_mode;
         key.g2p_tile = ctx->g2p_tile;
         key.tile_cap = ctx->tile_cap;
-        key.seg_cap = ctx->seg_cap;
         key.fuse = use_fused(ctx) ? 1 : 0;
         key.params_version = ctx->params_version;
         key.flags = flags & (EMPM_ROLLOUT_RESUME | EMPM_ROLLOUT_KEEP | EMPM_ROLLOUT_TAPE);
@@ -1756,7 +1755,6 @@ static SegGraphKey segment_key(const EmpmCtx* ctx) {
     memset(&k, 0, sizeof(k));
     k.epoch = ctx->epoch;
     k.params_version = ctx->params_version;
-    k.seg_cap = ctx->seg_cap;
     k.p2g_mode = ctx->p2g_mode;
     k.sort_every = ctx->sort_every;
     k.n = ctx->n_particles;
