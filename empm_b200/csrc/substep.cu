@@ -56,6 +56,7 @@ __global__ void k_prepare(const float* E, const float* nu, float* mu, float* lam
     if (density && vol && x) x[p].w = density[p] * vol[p];
 }
 
+template <bool TAPE>
 __global__ void k_debug_stress(const float* Ft9, float* mu, float* lam, float* ys, float dt, MaterialScalars ms,
                                float* F9, float* S9, int n) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -63,7 +64,7 @@ __global__ void k_debug_stress(const float* Ft9, float* mu, float* lam, float* y
     M3 Ft;
     for (int i = 0; i < 9; ++i) Ft.m[i] = Ft9[9 * p + i];
     float m = mu[p], l = lam[p], y = ys[p];
-    const ConstitutiveOut co = constitutive(Ft, m, l, y, dt, ms);
+    const ConstitutiveOut co = TAPE ? constitutive_general(Ft, m, l, y, dt, ms) : constitutive(Ft, m, l, y, dt, ms);
     mu[p] = m; lam[p] = l; ys[p] = y;
     for (int i = 0; i < 9; ++i) { F9[9 * p + i] = co.F.m[i]; S9[9 * p + i] = co.tau.m[i]; }
 }
@@ -1250,8 +1251,9 @@ extern "C" int empm_last_error(EmpmCtx* ctx, char* buf, int len) {
     return EMPM_OK;
 }
 
-extern "C" int empm_debug_stress(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
-                                 float* yield_stress, float dt, float* F_out9, float* stress_out9, int n, void* stream) {
+template <bool TAPE>
+static int debug_stress(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
+                        float* yield_stress, float dt, float* F_out9, float* stress_out9, int n, void* stream) {
     EmpmCtx* ctx = nullptr;
     int rc = validate_params(nullptr, params);
     if (rc) return rc;
@@ -1265,10 +1267,21 @@ extern "C" int empm_debug_stress(const EmpmModelParams* params, const float* F_t
     ms.xi = params->xi;
     ms.plastic_viscosity = params->plastic_viscosity;
     ms.alpha = params->alpha;
-    k_debug_stress<<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(F_trial9, mu, lam, yield_stress, dt, ms,
+    k_debug_stress<TAPE><<<blocks_for(n, 128), 128, 0, (cudaStream_t)stream>>>(F_trial9, mu, lam, yield_stress, dt, ms,
                                                                          F_out9, stress_out9, n);
     CK(cudaGetLastError(), "k_debug_stress");
     return EMPM_OK;
+}
+
+extern "C" int empm_debug_stress(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
+                                 float* yield_stress, float dt, float* F_out9, float* stress_out9, int n, void* stream) {
+    return debug_stress<false>(params, F_trial9, mu, lam, yield_stress, dt, F_out9, stress_out9, n, stream);
+}
+
+extern "C" int empm_debug_stress_tape(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
+                                      float* yield_stress, float dt, float* F_out9, float* stress_out9, int n,
+                                      void* stream) {
+    return debug_stress<true>(params, F_trial9, mu, lam, yield_stress, dt, F_out9, stress_out9, n, stream);
 }
 
 extern "C" int empm_ctx_grid(EmpmCtx* ctx, float** momentum, float** velocity) {

@@ -634,9 +634,12 @@ int  empm_debug_stress_adjoint(const EmpmModelParams* params, const float* F_tri
 /* Return map + Kirchhoff stress of the material switch for n particles, on
  * the device, in the reference's [N,3,3] row-major layout: the body of
  * compute_stress_from_F_trial (mpm_utils.py:602-665). mu, lam, yield_stress
- * are updated in place as the reference's return maps do. */
+ * are updated in place as the reference's return maps do. The update of sorted
+ * rollouts; _tape: that of single substeps, tapes and EMPM_ROLLOUT_TAPE. */
 int  empm_debug_stress(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
                        float* yield_stress, float dt, float* F_out9, float* stress_out9, int n, void* stream);
+int  empm_debug_stress_tape(const EmpmModelParams* params, const float* F_trial9, float* mu, float* lam,
+                            float* yield_stress, float dt, float* F_out9, float* stress_out9, int n, void* stream);
 
 /* Per-kernel timing with CUDA events on the launch stream (stream path of
  * empm_substep / empm_rollout only; graph replays are not instrumented).
