@@ -65,10 +65,10 @@ class PackedGrad:
         return self.v4[:, :3].clone()
 
     def C_mat(self) -> Tensor:
-        return _f9_unpack(self.C, self.n).clone()
+        return _f9_unpack(self.C, self.n)
 
     def F_mat(self) -> Tensor:
-        return _f9_unpack(self.F, self.n).clone()
+        return _f9_unpack(self.F, self.n)
 
 
 @dataclass

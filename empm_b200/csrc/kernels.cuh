@@ -788,7 +788,7 @@ __device__ __forceinline__ void p2g_cells(CellScatter<true, NT>& sh, bool valid,
 
 // order: NULL for particles sorted by cell, else the order that makes them so (single
 // substeps, k_order_*). Reading the state through it costs 15 sectors a particle: 500k
-// in random order 71.9 us (jelly), 82.6 (sand), against 42 us sorted.
+// in random order 74 us (jelly), 83 (sand), against 42 us sorted.
 template <int NT, int MAT, int MINB, bool TAPE>
 __global__ void __launch_bounds__(NT, MINB) k_p2g_cells(ParticleArrays P, MaterialArrays M, F9Planes Fe, Launch L,
                                                         float4* grid, unsigned char* flags, const int* order) {
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(NT, MINB) k_g2p2g_store(MaterialArrays M, Laun
         f9_store(a.cur.C, p, m3_zero());
         f9_store(a.cur.F, p, m3_identity());
     }
-    p2g_cells<MAT, true>(sh, valid, c, *c.step, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, a.fe_cur,
+    p2g_cells<MAT, TAPE>(sh, valid, c, *c.step, M, p, nx, xm.w, o.v, o.C, Fn, ah.mu, ah.lam, ah.ys, ah.vol, a.fe_cur,
                    a.cur.v, mom, flags);
 }
 
