@@ -1,8 +1,8 @@
 // pairs.cuh — arithmetic on pairs of floats.
 //
 // fma / mul / add.rn.f32x2 (sm_100) do two single-precision operations in one
-// instruction, each rounded as the scalar one is. The particle kernels are
-// bound by instruction issue (63 % of the issue slots, FMA pipe 32 %), so the
+// instruction, each rounded as the scalar one is. The particle kernels were
+// bound by instruction issue (63 % of the issue slots; 49 % with pairs), so the
 // stencil sums carry a vector's x and y as one pair.
 #pragma once
 #include "mat3.cuh"

@@ -2,9 +2,9 @@
 // entry is filled in. Only the time, the gates and the points that move with
 // their velocity differ between the substeps of a call without host callbacks
 // (mpm_solver_diff.py:186-291, 795-801 of the reference evaluate them once per
-// substep in Python, as this framework did: 25 us a substep with five
-// colliders, more than the substep's kernels take at 20k particles; here under
-// 0.2 us, the copy of the entry's 2.4 KB).
+// substep in Python, as this framework did: 20 us a substep with one collider, 60
+// with five, more than the substep's kernels take at 20k particles; here 0.3 us,
+// the copy of the entry's 2.4 KB).
 #include <cstring>
 
 #include "../../include/empm_b200.h"

@@ -131,12 +131,12 @@ static void free_sorted(SortedBuffers& sb) {
 // From this many particles on a single substep's P2G goes over the particles in cell
 // order (k_order_*, then the per-cell scatter with the state read through the order)
 // instead of in the caller's (k_p2g_direct, bound by its 27 reductions per particle).
-// Particles in random order, the P2G with its ordering, us:
-//   n       16k    30k    60k   120k   250k   500k    1M
-//   direct  17.4   25.3   39.5   80.3  163.6  284.5  462.2
-//   order   15.6   15.5   23.2   33.1   60.2  106.3  214.7
-// Below the line the calls wait on the host (90 us each from Python) and three more
-// launches would cost it 7 us. More than 64 cells per particle keep the direct kernel:
+// Particles in random order, the P2G with its ordering, us (sand; jelly 2 to 10 % less):
+//   n        66k   120k   250k   500k    1M
+//   direct  68.3  119.7  123.7  233.3  468.8
+//   order   39.8   48.7   68.4  107.0  216.9
+// Below the line the calls wait on the host (80 us each from Python; 16k particles: P2G
+// 17.4 us direct, 15.6 in order) and three more launches would cost it 7 us. More than 64 cells per particle keep the direct kernel:
 // the counts would outgrow the particles' state. The G2P stays in the caller's order
 // (500k: 57.8 us; through the order 81, its scattered stores).
 constexpr int kOrderMin = 65536;
@@ -618,8 +618,9 @@ static ParticleArrays particle_arrays(float* base, int n) {
 // Threads per block of the P2G kernels: the kernel's usual size, or 64 when
 // that would leave fewer than two blocks per SM (small instances would
 // otherwise run on a fraction of the SMs; measured 16.7 -> 15.0 us for 20k
-// particles; G2P measured no better). The kernels use no block-wide
-// synchronisation, so any multiple of the warp size works.
+// particles; G2P measured no better). For the direct kernels, which use no block-wide
+// synchronisation; the per-cell ones have barriers and their size as a template
+// parameter (EMPM_CELL_LAUNCH), and take from here only whether particles are few.
 static int particle_threads(const EmpmCtx* ctx, long long n, int usual) {
     return blocks_for(n, usual) >= 2LL * ctx->sm_count ? usual : 64;
 }
